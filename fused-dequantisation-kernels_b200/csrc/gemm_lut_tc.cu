@@ -94,14 +94,6 @@ __device__ __forceinline__ uint32_t ring32(uint32_t addr) {
   return v;
 }
 
-template <bool FP16>
-__device__ __forceinline__ uint32_t mul_pair(uint32_t a, uint32_t b) {  // two 16-bit products, rounded to nearest
-  uint32_t d;
-  if constexpr (FP16) asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-  else asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-  return d;
-}
-
 // The 16 elements (eight bf16 pairs) of one row's share of a 64-block, in element order.
 // w: the row's code words -- 4 bits: two words; 8 bits: four; 2 bits: one; 1 bit: the two
 // bytes starting at byte 2 * HH of w[0]; 3 bits: the 48-bit field group starting at bit 48 * HH

@@ -96,6 +96,14 @@ __device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], 
   }
 }
 
+template <bool FP16>
+__device__ __forceinline__ uint32_t mul_pair(uint32_t a, uint32_t b) {  // two 16-bit products, rounded to nearest
+  uint32_t d;
+  if constexpr (FP16) asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  else asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
+
 template <int I>
 __device__ __forceinline__ uint32_t word_of(const uint4& v) {
   if constexpr (I == 0) return v.x;
