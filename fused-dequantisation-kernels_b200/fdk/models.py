@@ -184,9 +184,16 @@ class QuantisedLinear(nn.Module):
         n_codes = 2**c.bits
         if lut is not None:
             assert lut.ndim == 1 and lut.shape[0] <= n_codes, f"lut must have at most {n_codes} entries, got {lut.shape[0]}"
-            lut = nn.functional.pad(lut, (0, n_codes - lut.shape[0]), value=lut[-1])
         else:
             lut = torch.linspace(-1, 1, steps=n_codes, device=device, dtype=weight.dtype)  # uniform [-1, 1]
+        if native.can_quantise(weight, c.bits, c.block_size, lut):
+            # one kernel, the same bytes as the operations below
+            source = weight.detach()
+            scale = None
+            if c.bits <= 2:  # a mean depends on the order of its sum: the framework's own
+                scale = source.unflatten(-1, (-1, c.block_size)).abs().mean(dim=-1).clamp_min_(1e-12)
+            return cls(*weight.T.shape, *native.quantise(source, c.bits, c.block_size, lut, scale), kernel=c.kernel)
+        lut = nn.functional.pad(lut, (0, n_codes - lut.shape[0]), value=lut[-1])
 
         # one scale per block_size run of the input dimension
         blocks = weight.unflatten(-1, (-1, c.block_size))

@@ -103,6 +103,10 @@ _SIGNATURES = {
     "fdk_status_string": (ctypes.c_char_p, [ctypes.c_int]),
     "fdk_last_error_detail": (ctypes.c_char_p, []),
     "fdk_tiled_size": (ctypes.c_int, [ctypes.c_int] * 3 + [ctypes.POINTER(ctypes.c_size_t)]),
+    "fdk_quantise": (
+        ctypes.c_int,
+        [ctypes.c_void_p] + [ctypes.c_int] * 5 + [ctypes.c_void_p, ctypes.c_int] + [ctypes.c_void_p] * 5,
+    ),
     "fdk_repack": (ctypes.c_int, [ctypes.c_void_p] * 2 + [ctypes.c_int] * 4 + [ctypes.c_void_p] * 2),
     "fdk_unpack": (ctypes.c_int, [ctypes.c_void_p] + [ctypes.c_int] * 4 + [ctypes.c_void_p] * 3),
     "fdk_dequantise": (ctypes.c_int, [ctypes.c_void_p] * 3 + [ctypes.c_int] * 5 + [ctypes.c_void_p] * 2),
@@ -195,6 +199,41 @@ def tiled_size(n: int, k: int, bits: int) -> int:
     out = ctypes.c_size_t(0)
     check(lib().fdk_tiled_size(n, k, bits, ctypes.byref(out)))
     return out.value
+
+
+def can_quantise(weight: Tensor, bits: int, block_size: int, lut: Tensor) -> bool:
+    """Whether `quantise` takes this weight and codebook: plain contiguous 16-bit CUDA tensors of one
+    type (nothing that a tensor subclass or autograd would have to see) and a scale block that
+    is a group of lanes of the kernel."""
+    return (
+        type(weight) in (Tensor, torch.nn.Parameter) and type(lut) in (Tensor, torch.nn.Parameter, torch.nn.Buffer)
+        and weight.is_cuda and lut.device == weight.device and weight.dtype == lut.dtype
+        and weight.dtype in (torch.bfloat16, torch.float16) and weight.ndim == 2 and weight.numel() > 0
+        and lut.ndim == 1 and lut.shape[0] > 0 and not (lut.requires_grad and torch.is_grad_enabled())
+        and bits in (1, 2, 3, 4, 8) and block_size in (8, 16, 32, 64, 128, 256) and weight.shape[1] % block_size == 0
+        and max(weight.shape) < 2**31 and weight.is_contiguous() and weight.data_ptr() % 16 == 0
+    )
+
+
+def quantise(weight: Tensor, bits: int, block_size: int, lut: Tensor, scale: Tensor | None) -> tuple[Tensor, Tensor, Tensor]:
+    """Dense weight [n, k] and codebook -> packed codes, block scales, byte table (reference layout).
+    The scales are the blocks' largest magnitudes, or those given."""
+    _require_cuda(weight, lut)
+    n, k = weight.shape
+    dev, dt = weight.device, weight.dtype
+    codes = torch.empty((n, k * bits // 8), dtype=torch.uint8, device=dev)
+    table = torch.empty((8, 1) if bits == 3 else (256, 8 // bits), dtype=dt, device=dev)
+    out_scale = torch.empty((n, k // block_size), dtype=dt, device=dev) if scale is None else scale
+    lut = lut.detach().contiguous()
+    with torch.cuda.device(dev):
+        check(
+            lib().fdk_quantise(
+                weight.data_ptr(), n, k, bits, block_size, dtype_code(dt), lut.data_ptr(), lut.shape[0],
+                None if scale is None else scale.data_ptr(), codes.data_ptr(),
+                out_scale.data_ptr() if scale is None else None, table.data_ptr(), _stream(),
+            )
+        )
+    return codes, out_scale, table
 
 
 def repack(codes: Tensor, scale: Tensor, n: int, k: int, bits: int, block_size: int) -> Tensor:

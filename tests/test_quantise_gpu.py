@@ -1,0 +1,62 @@
+"""The quantiser kernel against the sequence of torch operations that defines it, byte for byte."""
+
+import pytest
+import torch
+
+from fdk import models, native
+
+pytestmark = pytest.mark.gpu
+
+
+def by_torch(weight, config, lut):
+    """`QuantisedLinear.create` of the same weight without the kernel: in 16 bits, on the same GPU."""
+    can, native.can_quantise = native.can_quantise, lambda *a: False
+    try:
+        return models.QuantisedLinear.create(weight, config, lut=lut)
+    finally:
+        native.can_quantise = can
+
+
+@pytest.mark.parametrize("bits", [1, 2, 3, 4, 8])
+@pytest.mark.parametrize("n,k,block", [(1, 64, 64), (5, 192, 64), (64, 8, 8), (3, 1024, 256), (300, 640, 32), (513, 2048, 128)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_create_bytes_equal_torch(bits, n, k, block, dtype):
+    gen = torch.Generator(device="cuda").manual_seed(n + k + bits)
+    w = (torch.randn((n, k), generator=gen, device="cuda") * k**-0.5).to(dtype)
+    w.view(-1)[:: 97] = 0.0
+    w[-1, : block] = 0.0  # a block of zeros: its scale is the lower limit
+    short = torch.sort(torch.randn(max(2, 2**bits - 1), generator=gen, device="cuda"))[0].to(dtype)  # one entry short from 2 bits on
+    for lut in (None, models.kmeans_like_codebook(bits).to("cuda", dtype) if bits < 8 else None, short, short.flip(0)):
+        config = models.QuantisationConfig(bits, block)
+        assert native.can_quantise(w, bits, block, short)
+        got, want = models.QuantisedLinear.create(w, config, lut=lut), by_torch(w, config, lut)
+        assert torch.equal(got.weight_data, want.weight_data)
+        assert torch.equal(got.scale.view(torch.int16), want.scale.view(torch.int16))
+        assert torch.equal(got.lut.view(torch.int16), want.lut.view(torch.int16))
+        assert got.lut.shape == want.lut.shape and got.scale.shape == want.scale.shape
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_every_quotient_class(dtype):
+    """All 16-bit patterns as weights (subnormals, infinities and NaN among them), in blocks whose scales
+    span the type's range: the reciprocal form of the quotient and the division agree."""
+    patterns = torch.arange(65536, device="cuda", dtype=torch.int32).to(torch.int16).view(dtype)
+    gen = torch.Generator(device="cuda").manual_seed(0)
+    w = torch.cat([patterns.view(-1, 64), patterns[torch.randperm(65536, generator=gen, device="cuda")].view(-1, 64)])
+    w = torch.cat([w, torch.where(w.isfinite(), w, torch.zeros_like(w))])
+    config = models.QuantisationConfig(8, 64)
+    got, want = models.QuantisedLinear.create(w, config), by_torch(w, config, None)
+    assert torch.equal(got.weight_data, want.weight_data)
+    assert torch.equal(got.scale.isnan(), want.scale.isnan())
+    assert torch.equal(got.scale.nan_to_num(), want.scale.nan_to_num())
+
+
+def test_other_weights_keep_the_general_path():
+    w = torch.randn((64, 128), device="cuda").bfloat16()
+    lut = torch.linspace(-1, 1, 16, device="cuda", dtype=torch.bfloat16)
+    assert native.can_quantise(w, 4, 64, lut)
+    for bad in (w.t(), w[:, 1:65], w.float(), w.view(2, 32, 128), w[:0]):
+        assert not native.can_quantise(bad, 4, 64, lut)
+    assert not native.can_quantise(w, 4, 48, lut) and not native.can_quantise(w, 5, 64, lut)
+    t = models.QuantisedLinear.create(w.t().contiguous().t(), models.QuantisationConfig(4, 64))
+    assert torch.equal(t.weight_data, models.QuantisedLinear.create(w, models.QuantisationConfig(4, 64)).weight_data)
