@@ -1,27 +1,37 @@
 // Fused dequantise + GEMM for batches of 17 and more rows, on the fifth-generation tensor
 // cores:  out[m, n] = x[m, k] . W[n, k]^T  with W = bf16(table value * block scale), the
-// reference's dense W (src/fdk/kernels.py:23-24) bit for bit (fp16(...) for fp16 inputs), built tile by tile in shared
-// memory and never written to HBM.
+// reference's dense W (src/fdk/kernels.py:23-24) bit for bit (fp16(...) for fp16 inputs), built
+// block by block in tensor memory and never written to HBM.
 //
-// One CTA per 128 weight rows (the MMA M dimension; the batch is the MMA N dimension, so a
-// weight tile is dequantised once for the whole batch).  Six warps, specialised:
-//   warp 0      copy producer: per 64-column block, the [batch, 64] slice of x by a tiled TMA
-//               load (128-byte swizzle) into a ring of stages, and the two code slabs of the
-//               tile by cp.async.bulk -- with the stage where a slab holds one block (4 and 8
-//               bits), into a two-slot ring of their own where it holds two or four (1, 2,
-//               3 bits); completion on mbarriers;
-//   warps 2..9  dequantise: code bytes -> replicated table lookup -> multiply by the
-//               block scale in bf16 -> the 128 x 64 bf16 A tile of the stage, written in the
-//               K-major 128-byte-swizzled layout the MMA reads; afterwards the epilogue;
-//   warp 1      one thread issues tcgen05.mma (M = 128, N = batch padded to 16, K = 16, four
-//               per block) accumulating in tensor memory, and tcgen05.commit hands the stage
-//               back to the producer; it also owns the tensor-memory allocation.
-// Epilogue: tcgen05.ld brings the fp32 accumulators to registers (one tile row per thread),
-// converted to bf16 and stored transposed into out[batch, n].
-// Every barrier wait is bounded; a wait that runs out sets a status bit, and the kernel still
-// frees its tensor memory and returns.
+// Persistent, one CTA per SM.  The product is cut into tiles of 128 weight rows (MMA M) by up to
+// 256 batch rows (MMA N); the slabs of all tiles form one sequence, of which each CTA owns a
+// contiguous range, so every SM has the same work whatever the sizes.  A tile that is cut by a
+// range boundary belongs to the CTA with its first slabs; the others park their fp32 sums in the
+// workspace.  24 warps, specialised:
+//   warps 0..15  dequantise, in four sets of four warps; set s takes the 64-column blocks
+//                s, s + 4, ...: code bytes from shared memory -> replicated table lookup ->
+//                times the block scale -> tcgen05.st into the stage's A tile in TENSOR memory;
+//   warps 16..19 epilogue of a tile, while the next one is being computed (the last tile of
+//                a CTA, when the dequantising warps have nothing left to do, is shared with them);
+//   warps 20, 21 code slabs by cp.async.bulk, into a ring of their own;
+//   warp 22      x by tiled TMA loads (tensor map, 128-byte swizzle, no multicast);
+//   warp 23      allocates tensor memory; one thread issues tcgen05.mma (A from tensor memory,
+//                x from shared memory) and tcgen05.commit hands the stage back.
+// What bounds it: up to about 128 batch rows the dequantising warps (a block of 128 x 64 weights takes
+// ~750 warp instructions, ~190 cycles of four schedulers, and ~170 shared-memory wavefronts) and the
+// latency of the single threads that issue copies and MMAs (a barrier read queues behind the lookups:
+// 110 to 190 cycles); above, the tensor pipe (2 N cycles a block).  A in tensor memory keeps both
+// the store of the tile and the MMA's reads of it out of shared memory, and its MMAs of
+// small N are faster (a block at N = 32 takes 68 cycles, 161 with A in shared memory).  Before (A in
+// shared memory, eight dequantising warps, a tile per CTA) and now, 4 bits: 48 rows of 11264 x 3072 23.1 ->
+// 12.0 us; 2048 rows of 28672 x 4096 791 -> 370 us (1.30 PFLOP/s).  Tried and not kept: groups
+// of four blocks per copy, barrier and stage (18.4 us at 32 rows of 8192^2 against 16.7: a set
+// then waits for a whole group, and the larger stages leave fewer of them).
+// Every wait is bounded; one that runs out sets a status bit, and the kernel still frees its
+// tensor memory and returns.
 #include <cuda.h>
 
+#include <cmath>
 #include <cstring>
 
 #include "fdk_common.cuh"
@@ -30,32 +40,41 @@
 namespace fdk {
 namespace {
 
-constexpr int kTcDequantWarps = 8;
-constexpr int kTcThreads = 64 + 32 * kTcDequantWarps;
-constexpr int kTcMaxSplits = 8;
+constexpr int kTcDequantWarps = 16;
+constexpr int kTcEpilogueWarps = 4;
+constexpr int kTcCodeWarps = 2;
+constexpr int kTcWarps = kTcDequantWarps + kTcEpilogueWarps + kTcCodeWarps + 2;
+constexpr int kTcXWarp = kTcWarps - 2, kTcMmaWarp = kTcWarps - 1, kTcFirstCodeWarp = kTcXWarp - kTcCodeWarps;
+constexpr int kTcThreads = 32 * kTcWarps;
 constexpr int kTcTileRows = 128;
-constexpr int kTcMaxStages = 4;
+constexpr int kTcMaxBatch = 256;     // MMA N limit
+constexpr int kTcMaxStages = 8;
+constexpr int kTcMaxCodeSlots = 16;
+constexpr int kTcTmemColumns = 512;
+constexpr int kTcFlagsPerRank = (kTcMaxBatch / 16) * 4;  // 16 batch columns x 32 weight rows each
+// rows of the lookup table 256 bytes apart: a lookup address is one PRMT.  8 bits: no room beside
+// 256 batch rows and four slabs
+template <int BITS>
+constexpr bool kTcWideTable = BITS == 1 || BITS == 2 || BITS == 4;
 constexpr int kTcStatusTimeout = 1;
 constexpr int kTcStatusSmemLayout = 2;
 
 struct TcParams {
   const uint8_t* tiled;
-  const void* lut;   // device byte table, or null when it travels in the parameters
+  const void* lut;        // device byte table, or null when it travels in the parameters
   uint16_t* out;
-  int* status;       // device-side error bits
-  int m, m_pad, n, k;
-  int row_tiles;     // 64-row tiles of the tiled buffer
-  int k_blocks;      // k / 64
-  int stages;
-  int splits;        // CTAs sharing one 128-row tile, each with a contiguous range of 64-column blocks
-  float* partial;    // [tile][split - 1][m_pad][128] fp32 sums of the non-owning CTAs
-  int* flags;        // [tile][kTcMaxSplits] tag of the last published partial
-  int* uses;         // [tile] how often the tile has been finished through this workspace
-  uint32_t tmem_cols;
-  uint32_t smem_base, table_addr, bar_addr, tmem_slot_addr;
-  uint32_t a_addr[kTcMaxStages], b_addr[kTcMaxStages], c_addr[kTcMaxStages];
-  int k_slabs;            // slabs per 64-row tile
-  uint32_t cc_addr[2];    // code slots of the formats whose slabs span several blocks
+  int* status;            // device-side error bits
+  int m, n, n_tile;       // batch rows, weight rows, batch rows of a tile (multiple of 16)
+  int m_tiles, tiles;     // batch tiles; all tiles (the batch tile varies fastest)
+  int row_tiles;          // 64-row tiles of the tiled buffer
+  int k_blocks, k_slabs;  // k / 64; slabs per 64-row tile
+  int stages_log2, code_slots;
+  int acc_slots;          // accumulators in tensor memory: 2 where both fit beside the A stages
+  int split;              // ranges may cut tiles
+  float* partial;         // [rank][n_tile][128] fp32 sums of a CTA that does not own its first tile
+  int* flags;             // [rank][column sixteenth][row quarter] 1: published; the reader clears it again
+  uint32_t smem_base, table_addr, bar_addr;
+  uint32_t b_addr[kTcMaxStages], c_addr[kTcMaxCodeSlots];
 };
 
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
@@ -64,23 +83,38 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
       "l"(map), "r"(c0), "r"(c1), "r"(bar)
       : "memory");
 }
-
-// Shared-memory matrix descriptor: K-major, 128-byte swizzle, 8-row groups 1024 bytes apart.
-__device__ __forceinline__ uint64_t umma_desc(uint32_t addr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((addr & 0x3FFFFu) >> 4);        // start address
-  d |= (uint64_t)1 << 16;                        // leading byte offset (unused with swizzle)
-  d |= (uint64_t)(1024 >> 4) << 32;              // stride byte offset
-  d |= (uint64_t)1 << 46;                        // descriptor version
-  d |= (uint64_t)2 << 61;                        // SWIZZLE_128B
-  return d;
+// One thread of a converged warp.  The warps that issue copies and MMAs run their loops with all
+// lanes and only issue under this predicate: addresses and descriptors, which those instructions
+// take from uniform registers, then stay there (in a branch on the lane number each MMA
+// cost ~160 cycles of register moves: 8192^2, 32 rows: 30.5 us).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+__device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
+               "r"(bytes), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void mbar_expect(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+// Shared-memory matrix descriptor but for the address (its bits 4..17 go to bits 0..13): K-major,
+// 128-byte swizzle (2 in bits 61..63), 8-row groups 1024 bytes apart (bits 32..45, in 16-byte units; the
+// leading offset, bits 16..29, is unused with a swizzle), descriptor version 1 (bit 46).
+constexpr uint64_t kDescBase = ((uint64_t)2 << 61) | ((uint64_t)1 << 46) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 16);
+
+// D[tensor memory] (+)= A[tensor memory: one lane per row, two 16-bit elements per column] . B[shared]^T
+__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 
@@ -88,344 +122,494 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
+__device__ __forceinline__ void tmem_store16(uint32_t addr, const uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};" ::"r"(v[0]),
+      "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]),
+      "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(addr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_load16(uint32_t addr, uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(addr)
+      : "memory");
+}
+
 __device__ __forceinline__ uint32_t ring32(uint32_t addr) {
   uint32_t v;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
   return v;
 }
-
-// The 16 elements (eight bf16 pairs) of one row's share of a 64-block, in element order.
-// w: the row's code words -- 4 bits: two words; 8 bits: four; 2 bits: one; 1 bit: the two
-// bytes starting at byte 2 * HH of w[0]; 3 bits: the 48-bit field group starting at bit 48 * HH
-// of the 96 bits w[0..2].
-template <int BITS, int HH>
-__device__ __forceinline__ void decode_row16(const uint32_t (&w)[4], uint32_t lane_base, uint32_t (&v)[8]) {
-  if constexpr (BITS == 4) {
-    v[0] = lut32(entry_addr<4, 0>(w[0], lane_base)); v[1] = lut32(entry_addr<4, 1>(w[0], lane_base));
-    v[2] = lut32(entry_addr<4, 2>(w[0], lane_base)); v[3] = lut32(entry_addr<4, 3>(w[0], lane_base));
-    v[4] = lut32(entry_addr<4, 0>(w[1], lane_base)); v[5] = lut32(entry_addr<4, 1>(w[1], lane_base));
-    v[6] = lut32(entry_addr<4, 2>(w[1], lane_base)); v[7] = lut32(entry_addr<4, 3>(w[1], lane_base));
-  } else if constexpr (BITS == 8) {  // sixteen single lookups, merged in pairs
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      v[2 * i] = prmt<0x7610>(lut32(entry_addr<8, 0>(w[i], lane_base)), lut32(entry_addr<8, 1>(w[i], lane_base)));
-      v[2 * i + 1] = prmt<0x7610>(lut32(entry_addr<8, 2>(w[i], lane_base)), lut32(entry_addr<8, 3>(w[i], lane_base)));
-    }
-  } else if constexpr (BITS == 2) {  // one byte = four elements = one 8-byte entry
-    uint2 q;
-    q = lut64(entry_addr<2, 0>(w[0], lane_base)); v[0] = q.x; v[1] = q.y;
-    q = lut64(entry_addr<2, 1>(w[0], lane_base)); v[2] = q.x; v[3] = q.y;
-    q = lut64(entry_addr<2, 2>(w[0], lane_base)); v[4] = q.x; v[5] = q.y;
-    q = lut64(entry_addr<2, 3>(w[0], lane_base)); v[6] = q.x; v[7] = q.y;
-  } else if constexpr (BITS == 1) {  // one byte = eight elements = one 16-byte entry
-    uint4 q;
-    q = lut128(entry_addr<1, 2 * HH>(w[0], lane_base)); v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
-    q = lut128(entry_addr<1, 2 * HH + 1>(w[0], lane_base)); v[4] = q.x; v[5] = q.y; v[6] = q.z; v[7] = q.w;
-  } else {  // 3 bits: eight 6-bit pair fields, field f at bits [6f, 6f + 6) of the 96-bit group
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      constexpr int kStrideLog2 = 7;  // Table<3>::kStride
-      const int o = 6 * (8 * HH + i), wi = o >> 5, sh = o & 31;
-      uint32_t f;  // the field moved to bits 7..12: field * 128
-      if (sh + 6 <= 32) {
-        f = (sh >= kStrideLog2) ? (w[wi] >> (sh - kStrideLog2)) : (w[wi] << (kStrideLog2 - sh));
-      } else {
-        f = __funnelshift_r(w[wi], w[wi + 1], sh - kStrideLog2);
-      }
-      v[i] = lut32(lane_base + (f & (63u << kStrideLog2)));
-    }
-  }
+__device__ __forceinline__ uint2 ring64(uint32_t addr) {
+  uint2 v;
+  asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr) : "memory");
+  return v;
 }
 
+// A lane's tile row and the code words of it.  The tiled buffer gives the 16 elements [16 t, 16 t + 16)
+// of rows 16 r + g and 16 r + g + 8 to lane 4 g + t; here lane 4 g + t collects the whole block of
+// ONE row, 8 t + g of the warp's 32, because a tensor-memory lane is a row of A.  Fetching piece c
+// (16 elements) from all lanes at once would meet in a few banks, the rows being 64 and 512 bytes
+// apart, so lane l fetches piece c ^ x(l) in round c (x spreads what the bank bits of the row do
+// not) and the pieces are put in order by conditional swaps.
+template <int BITS>
+struct RowCodes {
+  static constexpr int kWords = BITS == 8 ? 4 : (BITS == 4 || BITS == 3) ? 2 : 1;  // words per piece
+  uint32_t w[4][kWords];
+
+  // slab: the 64-row slab of the lane's row; r: its 16-row sub-tile, half: row 8..15 of it; jb: block of the slab
+  __device__ __forceinline__ void load(uint32_t slab, int jb, int g, int r, int half, int x) {
+    using L = Layout<BITS>;
+    const uint32_t at = slab + (r * L::V * 32 + 4 * g) * 16;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const uint32_t lane_at = at + (uint32_t)((c ^ x) * 16);
+      if constexpr (BITS == 4) {
+        const uint2 q = ring64(lane_at + half * 8);
+        w[c][0] = q.x; w[c][1] = q.y;
+      } else if constexpr (BITS == 8) {
+        const uint4 q = ring128(lane_at + half * 512);
+        w[c][0] = q.x; w[c][1] = q.y; w[c][2] = q.z; w[c][3] = q.w;
+      } else if constexpr (BITS == 2) {
+        w[c][0] = ring32(lane_at + jb * 8 + half * 4);
+      } else if constexpr (BITS == 1) {
+        w[c][0] = ring32(lane_at + jb * 4) >> (16 * half);
+      } else {  // 3 bits: 12 bytes per block and lane, six of each row, in three 16-byte vectors
+        const int w0 = 3 * jb + half, w1 = w0 + 1;
+        const uint32_t a = ring32(lane_at + (w0 >> 2) * 512 + (w0 & 3) * 4), b = ring32(lane_at + (w1 >> 2) * 512 + (w1 & 3) * 4);
+        w[c][0] = __funnelshift_r(a, b, 16 * half);
+        w[c][1] = b >> (16 * half);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kWords; ++i) {
+      swap_if(x & 1, w[0][i], w[1][i]);
+      swap_if(x & 1, w[2][i], w[3][i]);
+      swap_if(x & 2, w[0][i], w[2][i]);
+      swap_if(x & 2, w[1][i], w[3][i]);
+    }
+  }
+  // Which piece lane 4 g + t of a warp fetches first.
+  __device__ static __forceinline__ int first_piece(int g, int t) {
+    if constexpr (BITS == 4) return ((g >> 1) & 1) | (t & 2);
+    else if constexpr (BITS == 8) return t;
+    else return g >> 1;
+  }
+  __device__ static __forceinline__ void swap_if(int cond, uint32_t& a, uint32_t& b) {
+    const uint32_t lo = cond ? b : a, hi = cond ? a : b;
+    a = lo;
+    b = hi;
+  }
+
+  // The 16 elements (eight pairs) of piece C, in element order, times the scale pair.
+  template <int C, bool FP16, bool WIDE>
+  __device__ __forceinline__ void decode(uint32_t lane_base, uint32_t s2, uint32_t (&v)[16], int at) const {
+    const uint32_t(&q)[kWords] = w[C];
+    if constexpr (BITS == 4) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        v[at + 4 * i] = lut32(entry_addr<4, 0, WIDE>(q[i], lane_base));
+        v[at + 4 * i + 1] = lut32(entry_addr<4, 1, WIDE>(q[i], lane_base));
+        v[at + 4 * i + 2] = lut32(entry_addr<4, 2, WIDE>(q[i], lane_base));
+        v[at + 4 * i + 3] = lut32(entry_addr<4, 3, WIDE>(q[i], lane_base));
+      }
+    } else if constexpr (BITS == 8) {  // sixteen single lookups, merged in pairs
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        v[at + 2 * i] = prmt<0x7610>(lut32(entry_addr<8, 0, WIDE>(q[i], lane_base)), lut32(entry_addr<8, 1, WIDE>(q[i], lane_base)));
+        v[at + 2 * i + 1] = prmt<0x7610>(lut32(entry_addr<8, 2, WIDE>(q[i], lane_base)), lut32(entry_addr<8, 3, WIDE>(q[i], lane_base)));
+      }
+    } else if constexpr (BITS == 2) {  // one byte = four elements = one 8-byte entry
+      const uint2 a = lut64(entry_addr<2, 0, WIDE>(q[0], lane_base)), b = lut64(entry_addr<2, 1, WIDE>(q[0], lane_base));
+      const uint2 c = lut64(entry_addr<2, 2, WIDE>(q[0], lane_base)), d = lut64(entry_addr<2, 3, WIDE>(q[0], lane_base));
+      v[at] = a.x; v[at + 1] = a.y; v[at + 2] = b.x; v[at + 3] = b.y;
+      v[at + 4] = c.x; v[at + 5] = c.y; v[at + 6] = d.x; v[at + 7] = d.y;
+    } else if constexpr (BITS == 1) {  // one byte = eight elements = one 16-byte entry
+      const uint4 a = lut128(entry_addr<1, 0, WIDE>(q[0], lane_base)), b = lut128(entry_addr<1, 1, WIDE>(q[0], lane_base));
+      v[at] = a.x; v[at + 1] = a.y; v[at + 2] = a.z; v[at + 3] = a.w;
+      v[at + 4] = b.x; v[at + 5] = b.y; v[at + 6] = b.z; v[at + 7] = b.w;
+    } else {  // 3 bits: eight 6-bit pair fields of a 48-bit group, each moved to bits 7..12 (times 128)
+      static_assert(BITS != 3 || Table<3>::kStride == 128, "field extraction assumes 128-byte table rows");
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int o = 6 * i;
+        const uint32_t f = o + 6 <= 32 ? (o >= 7 ? q[0] >> (o - 7) : q[0] << (7 - o))
+                           : o < 32    ? __funnelshift_r(q[0], q[1], o - 7)
+                           : o - 32 >= 7 ? q[1] >> (o - 39) : q[1] << (39 - o);
+        v[at + i] = lut32(lane_base + (f & (63u << 7)));
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[at + i] = mul_pair<FP16>(v[at + i], s2);
+  }
+};
+
+// Unit range of CTA `rank`: units are (tile, slab) pairs, a tile's slabs consecutive.
+__device__ __forceinline__ int range_begin(const TcParams& p, int rank) {
+  return p.split ? (int)((long long)p.tiles * p.k_slabs * rank / gridDim.x)
+                 : p.k_slabs * (int)((long long)p.tiles * rank / gridDim.x);
+}
+
+// Position in the unit sequence.  Stepped, not divided out: the warps that issue copies and MMAs
+// are single threads whose latency per block (two integer divisions cost ~300 cycles) was the
+// pace of the whole kernel: 8192^2, 32 rows: 33.7 us.
+struct Cursor {
+  int ks, mt, nt;
+  __device__ __forceinline__ Cursor(const TcParams& p, int unit) {
+    const int tile = unit / p.k_slabs;
+    ks = unit - tile * p.k_slabs;
+    nt = tile / p.m_tiles;
+    mt = tile - nt * p.m_tiles;
+  }
+  __device__ __forceinline__ bool next(const TcParams& p) {  // true at the first slab of a tile
+    if (++ks < p.k_slabs) return false;
+    ks = 0;
+    if (++mt == p.m_tiles) {
+      mt = 0;
+      ++nt;
+    }
+    return true;
+  }
+};
+
 template <int BITS, bool FP16>
-__global__ void __launch_bounds__(kTcThreads, 2)
+__global__ void __launch_bounds__(kTcThreads, 1)
     gemm_lut_tc_kernel(const __grid_constant__ TcParams p, const __grid_constant__ InlineLut<BITS> inl,
                        const __grid_constant__ CUtensorMap x_map) {
   using L = Layout<BITS>;
-  using T = Table<BITS>;
-  static_assert(T::kStride == 128, "3-bit field extraction assumes 128-byte table rows");
-  constexpr bool kOwnCodeRing = L::KSB > 1;  // slabs spanning several blocks live in a ring of their own
+  constexpr bool WIDE = kTcWideTable<BITS>;
+  using T = Table<BITS, WIDE>;
+  constexpr int KSB = L::KSB;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t raw = smem_addr(smem_raw);
   if (raw != p.smem_base) {
     if (threadIdx.x == 0) atomicOr(p.status, kTcStatusSmemLayout);
     return;
   }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int S = p.stages;
-  // barriers: tma_full[S], a_full[S], empty[S], accum_full
-  const uint32_t tma_full = p.bar_addr, a_full = p.bar_addr + 8 * S, empty = p.bar_addr + 16 * S,
-                 accum_full = p.bar_addr + 24 * S;
-  const uint32_t c_full = p.bar_addr + 8 * (3 * kTcMaxStages + 2), c_empty = c_full + 16;  // two slots each
-  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_raw + (p.tmem_slot_addr - raw));
-  const int tile = blockIdx.x / p.splits;         // 128 rows = 64-row tiles 2*tile, 2*tile + 1
-  const int sp = blockIdx.x - tile * p.splits;    // this CTA's share of the 64-column blocks
-  const int kb_begin = (int)((long long)p.k_blocks * sp / p.splits);
-  const int kb_end = (int)((long long)p.k_blocks * (sp + 1) / p.splits);
-  const int n_kb = kb_end - kb_begin;
-  const bool second_half = (2 * tile + 1) < p.row_tiles;
+  // x, the workspace and out are only touched after griddepcontrol.wait; codes and table are not
+  // written by the kernel before
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);  // uniform for the compiler
+  const int S = 1 << p.stages_log2;
+  const uint32_t full = p.bar_addr, empty = full + 8 * kTcMaxStages,
+                 c_full = empty + 8 * kTcMaxStages, c_empty = c_full + 8 * kTcMaxCodeSlots,
+                 acc_full = c_empty + 8 * kTcMaxCodeSlots, acc_empty = acc_full + 16, acc_last = acc_empty + 16, tmem_slot = acc_last + 8;
+  // Waits go to CTAs of lower block index, which the GPU starts first: rank r's successors in
+  // the unit sequence are the blocks before it.
+  const int rank = (int)gridDim.x - 1 - (int)blockIdx.x;
+  const int u0 = range_begin(p, rank), u1 = range_begin(p, rank + 1);
   bool timed_out = false;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) {
-      mbar_init(tma_full + 8 * s, 1);
-      mbar_init(a_full + 8 * s, kTcDequantWarps);  // one arrival per dequantising warp
+      mbar_init(full + 8 * s, 5);  // x has arrived, and the four warps of a set have stored A
       mbar_init(empty + 8 * s, 1);
     }
-    mbar_init(accum_full, 1);
-    for (int c = 0; c < 2; ++c) {
+    for (int c = 0; c < p.code_slots; ++c) {
       mbar_init(c_full + 8 * c, 1);
-      mbar_init(c_empty + 8 * c, kTcDequantWarps);
+      mbar_init(c_empty + 8 * c, KSB == 1 ? 4 : kTcDequantWarps);  // one set, or all
     }
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(acc_full + 8 * a, 1);
+      mbar_init(acc_empty + 8 * a, kTcEpilogueWarps);
+    }
+    mbar_init(acc_last, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  if (warp == 1) {  // tensor memory for the accumulator: 128 lanes x tmem_cols columns of fp32
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(p.tmem_slot_addr),
-                 "r"(p.tmem_cols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  if (warp >= 2) {
-    if (p.lut == nullptr) {
-      fill_table<BITS>(p.table_addr, 32 * kTcDequantWarps, [&](int i) { return inl.w[i]; }, threadIdx.x - 64);
-    } else {
-      fill_table<BITS>(p.table_addr, 32 * kTcDequantWarps,
-                       [&](int i) { return __ldg(reinterpret_cast<const uint32_t*>(p.lut) + i); }, threadIdx.x - 64);
-    }
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem_base = *tmem_slot;
+  // The copy producers are off; the others fill the table first.
+  if (warp < kTcFirstCodeWarp || warp == kTcMmaWarp) {
+    constexpr int kFillThreads = kTcThreads - 32 * (kTcCodeWarps + 1);
+    const int tid = warp == kTcMmaWarp ? kFillThreads - 32 + lane : threadIdx.x;
+    auto fill = [&](auto word) {
+      if constexpr (BITS == 4 || BITS == 2 || BITS == 1) fill_table_unrolled<BITS, WIDE, kFillThreads>(p.table_addr, word, tid);
+      else fill_table<BITS, WIDE>(p.table_addr, kFillThreads, word, tid);
+    };
+    if (p.lut == nullptr) fill([&](int i) { return inl.w[i]; });
+    else fill([&](int i) { return __ldg(reinterpret_cast<const uint32_t*>(p.lut) + i); });
+    if (warp == kTcMmaWarp) {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "r"((uint32_t)kTcTmemColumns)
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    asm volatile("bar.sync 1, %0;" ::"n"(kFillThreads) : "memory");
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  }
+  // All of tensor memory is allocated, so it starts at address 0; a constant keeps the MMAs' operands
+  // in uniform registers.
+  constexpr uint32_t tmem_base = 0;
+  const uint32_t acc_base = tmem_base + 32 * S;  // A stages of 32 columns, then the accumulators
+  auto blocks_of = [&](int ks) { return KSB == 1 ? 1 : min(KSB, p.k_blocks - ks * KSB); };
 
-  if (warp == 0) {
-    // ---------------- copy producer ----------------
-    if (lane == 0) {
-      const uint32_t code_bytes = L::kSlabBytes * (second_half ? 2 : 1);
-      const uint32_t x_bytes = (uint32_t)p.m_pad * 128;
-      auto load_codes = [&](int slab, uint32_t dst, uint32_t bar) {
-        const uint8_t* slab0 = p.tiled + ((size_t)(2 * tile) * p.k_slabs + slab) * L::kSlabBytes;
-        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-                     "l"(slab0), "r"((uint32_t)L::kSlabBytes), "r"(bar)
-                     : "memory");
-        if (second_half) {
-          const uint8_t* slab1 = p.tiled + ((size_t)(2 * tile + 1) * p.k_slabs + slab) * L::kSlabBytes;
-          asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                           dst + (uint32_t)L::kSlabBytes),
-                       "l"(slab1), "r"((uint32_t)L::kSlabBytes), "r"(bar)
-                       : "memory");
-        }
-      };
-      int loaded_slab = -1, slabs_loaded = 0;
-      for (int i = 0; i < n_kb; ++i) {
-        const int kb = kb_begin + i;
-        const int s = i % S;
-        const uint32_t phase = (i / S) & 1;
-        if constexpr (kOwnCodeRing) {
-          const int slab = kb / L::KSB;
-          if (slab != loaded_slab) {  // next slab into the slot freed two slabs ago
-            const int c = slabs_loaded & 1;
-            if (!mbar_wait(c_empty + 8 * c, ((slabs_loaded >> 1) & 1) ^ 1)) { timed_out = true; break; }
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(c_full + 8 * c), "r"(code_bytes) : "memory");
-            load_codes(slab, p.cc_addr[c], c_full + 8 * c);
-            loaded_slab = slab;
-            ++slabs_loaded;
-          }
-        }
-        if (!mbar_wait(empty + 8 * s, phase ^ 1)) { timed_out = true; break; }
-        const uint32_t bar = tma_full + 8 * s;
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
-                     "r"((kOwnCodeRing ? 0u : code_bytes) + x_bytes)
-                     : "memory");
-        if constexpr (!kOwnCodeRing) load_codes(kb, p.c_addr[s], bar);
-        tma_load_2d(p.b_addr[s], &x_map, kb * 64, 0, bar);
-      }
-    }
-  } else if (warp == 1) {
-    // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      // instruction descriptor: fp32 accumulate, A and B both bf16 (format 1) or both fp16
-      // (format 0), both K-major, N = m_pad, M = 128
-      constexpr uint32_t kFormat = FP16 ? 0u : 1u;
-      const uint32_t idesc = (1u << 4) | (kFormat << 7) | (kFormat << 10) | ((uint32_t)(p.m_pad >> 3) << 17) | ((128u >> 4) << 24);
-      for (int i = 0; i < n_kb; ++i) {
-        const int s = i % S;
-        const uint32_t phase = (i / S) & 1;
-        if (!mbar_wait(tma_full + 8 * s, phase)) { timed_out = true; break; }
-        if (!mbar_wait(a_full + 8 * s, phase)) { timed_out = true; break; }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        // one descriptor pair per stage; the four K = 16 slices of the 64-column block lie 32
-        // bytes apart, i.e. 2 in the descriptors' 16-byte address units
-        const uint64_t a_desc = umma_desc(p.a_addr[s]), b_desc = umma_desc(p.b_addr[s]);
+  // ---- epilogue of one tile segment [begin, end) of slabs, by `parts` warps per 32-row quarter ----
+  auto epilogue = [&](int tile, int begin, int end, uint32_t acc, int part, int parts) {
+    const int nt = tile / p.m_tiles, mt = tile - nt * p.m_tiles;
+    const int quarter = warp & 3;
+    const int row = nt * kTcTileRows + 32 * quarter + 8 * (lane & 3) + (lane >> 2);
+    const size_t slot = (size_t)p.n_tile * kTcTileRows;
+    const uint32_t taddr = acc + ((uint32_t)(quarter * 32) << 16);
+    const int tile_end = (tile + 1) * p.k_slabs;
+    int last_rank = rank;  // ranks rank + 1 .. last_rank hold the rest of the tile
+    if (begin == 0 && end < p.k_slabs)
+      while (range_begin(p, last_rank + 1) < tile_end) ++last_rank;
+    // flag of 16 columns of 32 rows: one warp publishes them, one consumes them
+    auto flag = [&](int of_rank, int c0) { return p.flags + of_rank * kTcFlagsPerRank + (c0 >> 4) * 4 + quarter; };
+    for (int c0 = 16 * part; c0 < p.n_tile; c0 += 16 * parts) {
+      uint32_t acc16[16];
+      tmem_load16(taddr + (uint32_t)c0, acc16);
+      const size_t at = (size_t)c0 * kTcTileRows + 32 * quarter + lane;
+      if (begin != 0) {
+        float* mine = p.partial + rank * slot + at;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          umma_bf16(tmem_base, a_desc + 2 * j, b_desc + 2 * j, idesc, (i > 0 || j > 0) ? 1u : 0u);
-        }
-        umma_commit(empty + 8 * s);  // the stage may be refilled once these MMAs have read it
-      }
-      umma_commit(accum_full);
-    }
-  } else {
-    // ---------------- dequantise, then epilogue ----------------
-    const int dw = warp - 2;          // 0..7: one of the eight 16-row sub-tiles each
-    const int g = lane >> 2, t = lane & 3;
-    const uint32_t lane_base = p.table_addr + T::lane_offset(lane);
-    int cur_slab = -1, slabs_seen = 0;
-    uint32_t code_slot = 0;
-    for (int i = 0; i < n_kb; ++i) {
-      const int s = i % S;
-      const uint32_t phase = (i / S) & 1;
-      const int kb = kb_begin + i;
-      const int jb = kOwnCodeRing ? kb % L::KSB : 0;  // block inside its slab
-      if constexpr (kOwnCodeRing) {
-        const int slab_index = kb / L::KSB;
-        if (slab_index != cur_slab) {
-          const int c = slabs_seen & 1;
-          if (!mbar_wait(c_full + 8 * c, (slabs_seen >> 1) & 1)) { timed_out = true; break; }
-          code_slot = p.cc_addr[c];
-          cur_slab = slab_index;
-          ++slabs_seen;
-        }
-      }
-      if (!mbar_wait(tma_full + 8 * s, phase)) { timed_out = true; break; }  // also: the stage's A tile is free
-      {
-        const int u = dw, half = u >> 2, r = u & 3;
-        if (!(half == 1 && !second_half)) {
-        const uint32_t slab = (kOwnCodeRing ? code_slot : p.c_addr[s]) + half * L::kSlabBytes;
-        const uint32_t scw = ring32(slab + L::kCodeBytes + jb * 128 + g * 16 + r * 4);
-        const uint32_t s_lo = prmt<0x1010>(scw, 0u), s_hi = prmt<0x3232>(scw, 0u);  // scale of row g / g+8 in both halves
-        uint32_t wg[4] = {0u, 0u, 0u, 0u}, wh[4] = {0u, 0u, 0u, 0u};  // code words of row g and of row g+8
-        if constexpr (BITS == 4) {
-          const uint4 c = ring128(slab + (r * 32 + lane) * 16);
-          wg[0] = c.x; wg[1] = c.y; wh[0] = c.z; wh[1] = c.w;
-        } else if constexpr (BITS == 8) {
-          const uint4 cg = ring128(slab + ((r * 2) * 32 + lane) * 16), ch = ring128(slab + ((r * 2 + 1) * 32 + lane) * 16);
-          wg[0] = cg.x; wg[1] = cg.y; wg[2] = cg.z; wg[3] = cg.w;
-          wh[0] = ch.x; wh[1] = ch.y; wh[2] = ch.z; wh[3] = ch.w;
-        } else if constexpr (BITS == 2) {  // the lane's 16 bytes: per block one word for row g, one for row g+8
-          const uint32_t at = slab + (r * 32 + lane) * 16 + jb * 8;
-          wg[0] = ring32(at);
-          wh[0] = ring32(at + 4);
-        } else if constexpr (BITS == 1) {  // per block one word: bytes 0,1 row g, bytes 2,3 row g+8
-          wg[0] = wh[0] = ring32(slab + (r * 32 + lane) * 16 + jb * 4);
-        } else {  // 3 bits: 48 bytes per lane in three 16-byte vectors, 12 bytes per block
+        for (int j = 0; j < 16; ++j) __stcg(mine + j * kTcTileRows, __uint_as_float(acc16[j]));
+      } else {
+        float v[16];
 #pragma unroll
-          for (int i3 = 0; i3 < 3; ++i3) {
-            const int wi = 3 * jb + i3;
-            wg[i3] = wh[i3] = ring32(slab + ((r * 3 + (wi >> 2)) * 32 + lane) * 16 + (wi & 3) * 4);
-          }
-        }
-        auto write_row = [&](auto hhc) {
-          constexpr int HH = decltype(hhc)::value;
-          uint32_t v[8];
-          decode_row16<BITS, HH>(HH == 0 ? wg : wh, lane_base, v);
-          const uint32_t sc = HH == 0 ? s_lo : s_hi;
-#pragma unroll
-          for (int i = 0; i < 8; ++i) v[i] = mul_pair<FP16>(v[i], sc);
-          const int row = 16 * u + g + 8 * HH;  // row % 8 == g
-          const uint32_t row_addr = p.a_addr[s] + row * 128;
-          const uint32_t c0 = ((2 * t) ^ g) * 16, c1 = ((2 * t + 1) ^ g) * 16;
-          asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(row_addr + c0), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
-          asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(row_addr + c1), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
-        };
-        write_row(std::integral_constant<int, 0>{});
-        write_row(std::integral_constant<int, 1>{});
-        }
-      }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic writes -> visible to the MMA
-      __syncwarp();
-      if (lane == 0) {
-        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(a_full + 8 * s) : "memory");
-        if constexpr (kOwnCodeRing) {  // last block read from this code slot: hand it back
-          if (jb == L::KSB - 1 || i == n_kb - 1) {
-            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(c_empty + 8 * ((slabs_seen - 1) & 1)) : "memory");
-          }
-        }
-      }
-    }
-    // epilogue (first four of these warps): each reads the 32 accumulator rows of its
-    // tensor-memory lane quarter.  A CTA that does not own the tile parks its fp32 sums in the
-    // workspace; the owner (share 0) adds the parked sums in share order and writes bf16.
-    if (dw < 4) {
-      if (!mbar_wait(accum_full, 0)) timed_out = true;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const int quarter = warp & 3;
-      const int row_in_tile = quarter * 32 + lane;
-      const int row = tile * kTcTileRows + row_in_tile;
-      int tag = 0;
-      if (p.splits > 1) tag = ld_relaxed_s32(p.uses + tile) + 1;
-      if (sp == 0 && p.splits > 1) {  // wait until every other share has been published
-        for (int o = 1; o < p.splits; ++o) {
-          unsigned long long t0 = 0;
-          for (uint32_t spin = 0;; ++spin) {
-            int f;
-            asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(f) : "l"(p.flags + tile * kTcMaxSplits + o) : "memory");
-            if (f == tag) break;
-            if ((spin & 255u) == 255u) {
-              unsigned long long now;
-              asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
-              if (t0 == 0) t0 = now;
-              else if (now - t0 > 2000000000ull) { timed_out = true; break; }
+        for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(acc16[j]);
+        if (last_rank > rank) {
+          for (int o = rank + 1 + lane; o <= last_rank; o += 32) {  // a lane per share
+            int* const f = flag(o, c0);
+            unsigned long long t0 = 0;
+            for (uint32_t spin = 0;; ++spin) {
+              int set;
+              asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(set) : "l"(f) : "memory");
+              if (set != 0) break;
+              if ((spin & 255u) == 255u) {
+                unsigned long long now;
+                asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+                if (t0 == 0) t0 = now;
+                else if (now - t0 > 2000000000ull) { timed_out = true; break; }
+              }
             }
+            *f = 0;
           }
-        }
-      }
-      for (int c0 = 0; c0 < p.m_pad; c0 += 16) {
-        uint32_t acc[16];
-        const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0;
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-            : "=r"(acc[0]), "=r"(acc[1]), "=r"(acc[2]), "=r"(acc[3]), "=r"(acc[4]), "=r"(acc[5]), "=r"(acc[6]), "=r"(acc[7]),
-              "=r"(acc[8]), "=r"(acc[9]), "=r"(acc[10]), "=r"(acc[11]), "=r"(acc[12]), "=r"(acc[13]), "=r"(acc[14]), "=r"(acc[15])
-            : "r"(taddr)
-            : "memory");
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (sp != 0) {
-          float* mine = p.partial + ((size_t)(tile * (p.splits - 1) + sp - 1) * p.m_pad + c0) * 128 + row_in_tile;
+          timed_out = __any_sync(0xffffffffu, timed_out);  // also orders the other lanes' reads after the flags
+          // in rank order; two shares' loads are in flight at a time
+          for (int o = rank + 1; o <= last_rank; o += 2) {
+            const float* theirs = p.partial + o * slot + at;
+            float t[32];
 #pragma unroll
-          for (int j = 0; j < 16; ++j) __stcg(mine + j * 128, __uint_as_float(acc[j]));
-        } else {
-          float v[16];
+            for (int j = 0; j < 16; ++j) t[j] = __ldcg(theirs + j * kTcTileRows);
+            if (o < last_rank) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(acc[j]);
-          for (int o = 1; o < p.splits; ++o) {  // share order; the sixteen loads of a share are independent
-            const float* theirs = p.partial + ((size_t)(tile * (p.splits - 1) + o - 1) * p.m_pad + c0) * 128 + row_in_tile;
-            float t[16];
-#pragma unroll
-            for (int j = 0; j < 16; ++j) t[j] = __ldcg(theirs + j * 128);
+              for (int j = 0; j < 16; ++j) t[16 + j] = __ldcg(theirs + slot + j * kTcTileRows);
+            }
 #pragma unroll
             for (int j = 0; j < 16; ++j) v[j] += t[j];
-          }
-          if (row < p.n) {
+            if (o < last_rank) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const int b = c0 + j;
-              if (b < p.m) p.out[(size_t)b * p.n + row] = from_float<FP16>(v[j]);
+              for (int j = 0; j < 16; ++j) v[j] += t[16 + j];
             }
           }
         }
-      }
-      if (p.splits > 1) {
-        __threadfence();
-        // the four epilogue warps meet on a named barrier, then one thread publishes
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        if (dw == 0 && lane == 0) {
-          if (sp != 0) {
-            asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p.flags + tile * kTcMaxSplits + sp), "r"(tag) : "memory");
-          } else {
-            p.uses[tile] = tag;  // the next use of this tile waits for tags one higher
-          }
+        if (row < p.n) {
+          const int b0 = mt * p.n_tile + c0;
+          uint16_t* dst = p.out + (size_t)b0 * p.n + row;
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (b0 + j < p.m) dst[(size_t)j * p.n] = from_float<FP16>(v[j]);
         }
       }
     }
+    if (begin != 0) {  // publish: no barrier, every warp vouches for its own columns
+      __syncwarp();
+      __threadfence();
+      const int c0 = 16 * (part + lane * parts);
+      if (c0 < p.n_tile) asm volatile("st.relaxed.gpu.global.s32 [%0], %1;" ::"l"(flag(rank, c0)), "r"(1) : "memory");
+    }
+  };
+  constexpr int kSets = kTcDequantWarps / 4;
+  // the CTA's last tile segment
+  const int last_tile = u1 > u0 ? (u1 - 1) / p.k_slabs : 0;
+  const int last_begin = max(u0 - last_tile * p.k_slabs, 0), last_end = u1 - last_tile * p.k_slabs;
+  const int segments = u1 > u0 ? last_tile - u0 / p.k_slabs + 1 : 0;
+  auto last_epilogue = [&](int part) {
+    if (!mbar_wait(acc_last, 0)) timed_out = true;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    epilogue(last_tile, last_begin, last_end, acc_base + (segments - 1) % p.acc_slots * p.n_tile, part, kSets + 1);
+  };
+
+  if (segments == 0) {
+    // more CTAs than units
+  } else if (warp >= kTcFirstCodeWarp && warp < kTcXWarp) {
+    // ---------------- code producer ----------------
+    // two warps, a slab each in turn: wait, expectation and two copies take one of them ~300 cycles
+    const int first = warp - kTcFirstCodeWarp;
+    int slot = first, phase = 0;
+    const size_t tile_bytes = (size_t)p.k_slabs * L::kSlabBytes;  // one 64-row tile
+    Cursor c(p, u0 + first);
+    for (int u = u0 + first; u < u1; u += kTcCodeWarps) {
+      const uint8_t* src = p.tiled + 2 * c.nt * tile_bytes + (size_t)c.ks * L::kSlabBytes;
+      const bool second = 2 * c.nt + 1 < p.row_tiles;
+      const uint32_t bar = c_full + 8 * slot, dst = p.c_addr[slot];
+      if (!mbar_wait(c_empty + 8 * slot, phase ^ 1)) { timed_out = true; break; }
+      if (elect_one()) {
+        mbar_expect(bar, (uint32_t)L::kSlabBytes * (second ? 2 : 1));
+        bulk_copy(dst, src, L::kSlabBytes, bar);
+        if (second) bulk_copy(dst + (uint32_t)L::kSlabBytes, src + tile_bytes, L::kSlabBytes, bar);
+      }
+      for (int i = 0; i < kTcCodeWarps; ++i) c.next(p);
+      if ((slot += kTcCodeWarps) >= p.code_slots) { slot -= p.code_slots; phase ^= 1; }
+    }
+  } else if (warp == kTcXWarp) {
+    // ---------------- x producer ----------------
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    int i = 0;
+    Cursor c(p, u0);
+    for (int u = u0; u < u1 && !timed_out; ++u, c.next(p)) {
+      const int nb = blocks_of(c.ks);
+      for (int jb = 0; jb < nb; ++jb, ++i) {
+        const int s = i & (S - 1);
+        const uint32_t dst = p.b_addr[s], bar = full + 8 * s;
+        if (!mbar_wait(empty + 8 * s, ((i >> p.stages_log2) & 1) ^ 1)) { timed_out = true; break; }
+        if (elect_one()) {
+          mbar_expect(bar, (uint32_t)p.n_tile * 128);
+          tma_load_2d(dst, &x_map, (c.ks * KSB + jb) * kBlock, c.mt * p.n_tile, bar);
+        }
+      }
+    }
+  } else if (warp == kTcMmaWarp) {
+    // ---------------- MMA issuer ----------------
+    // instruction descriptor: fp32 accumulate, A and B both bf16 (format 1) or both fp16
+    // (format 0), both K-major, N = n_tile, M = 128
+    constexpr uint32_t kFormat = FP16 ? 0u : 1u;
+    const uint32_t idesc = (1u << 4) | (kFormat << 7) | (kFormat << 10) | ((uint32_t)(p.n_tile >> 3) << 17) | ((128u >> 4) << 24);
+    int i = 0, ks = u0 % p.k_slabs;
+    for (int seg = 0, u = u0; seg < segments && !timed_out; ++seg) {
+      const int a = seg % p.acc_slots;
+      const uint32_t acc = acc_base + a * p.n_tile;
+      if (!mbar_wait(acc_empty + 8 * a, ((seg / p.acc_slots) & 1) ^ 1)) { timed_out = true; break; }
+      uint32_t accumulate = 0;
+      for (bool more = true; more && !timed_out;) {
+        const int nb = blocks_of(ks);
+        if (++ks == p.k_slabs) { ks = 0; more = false; }
+        if (++u == u1) more = false;
+        for (int jb = 0; jb < nb; ++jb, ++i) {
+          const int s = i & (S - 1);
+          const uint32_t parity = (i >> p.stages_log2) & 1;
+          const uint64_t b_desc = kDescBase | (p.b_addr[s] >> 4);
+          if (!mbar_wait(full + 8 * s, parity)) { timed_out = true; break; }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          // four K = 16 slices of the 64-column block: 8 columns of A, 32 bytes of x (2 in the
+          // descriptor's 16-byte units) apart
+          if (elect_one()) {
+            umma_f16_ts(acc, tmem_base + 32 * s, b_desc, idesc, accumulate);
+            umma_f16_ts(acc, tmem_base + 32 * s + 8, b_desc + 2, idesc, 1);
+            umma_f16_ts(acc, tmem_base + 32 * s + 16, b_desc + 4, idesc, 1);
+            umma_f16_ts(acc, tmem_base + 32 * s + 24, b_desc + 6, idesc, 1);
+            umma_commit(empty + 8 * s);  // the stage may be refilled once these MMAs have read it
+          }
+          accumulate = 1;
+        }
+      }
+      // the last segment has a barrier of its own, for the dequantising warps too, which have
+      // not followed acc_full's phases
+      if (elect_one()) umma_commit(seg + 1 < segments ? acc_full + 8 * a : acc_last);
+    }
+  } else if (warp >= kTcDequantWarps) {
+    // ---------------- epilogue ----------------
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    int u = u0;
+    for (int seg = 0; seg + 1 < segments; ++seg) {
+      const int tile = u / p.k_slabs, begin = u - tile * p.k_slabs;
+      const int a = seg % p.acc_slots;
+      if (!mbar_wait(acc_full + 8 * a, (seg / p.acc_slots) & 1)) timed_out = true;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      epilogue(tile, begin, p.k_slabs, acc_base + a * p.n_tile, 0, 1);
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(acc_empty + 8 * a);
+      u = (tile + 1) * p.k_slabs;
+    }
+    last_epilogue(kSets);
+  } else {
+    // ---------------- dequantise ----------------
+    const int set = warp >> 2, quarter = warp & 3;
+    const int g = lane >> 2, t = lane & 3;
+    const int r = 2 * (quarter & 1) + (t >> 1), half = t & 1;  // the lane's row: 32 quarter + 8 t + g
+    const int x = RowCodes<BITS>::first_piece(g, t);
+    const uint32_t slab_off = (quarter >> 1) * (uint32_t)L::kSlabBytes;
+    const uint32_t scale_off = slab_off + L::kCodeBytes + g * 16 + r * 4;
+    const uint32_t lane_base = p.table_addr + T::lane_offset(lane);
+    const uint32_t a_lane = tmem_base + ((uint32_t)(quarter * 32) << 16);
+    // Codes and scale pair of the set's next block -> its number in the CTA's sequence; -1 at the end.
+    // A warp may only skip the barriers of stages and code slots that it never uses: waiting
+    // for a phase while the one before it is still open would succeed at once.  Stages, and
+    // slots of slabs with one block, always belong to the same set (their number is a multiple
+    // of four); the other slabs are seen by every warp.
+    int u = KSB == 1 ? u0 + set : u0, slot = KSB == 1 ? set : 0, c_phase = 0;
+    int ks = KSB == 1 ? 0 : u0 % p.k_slabs, i = 0;
+    auto fetch = [&](RowCodes<BITS>& codes, uint32_t& s2) -> int {
+      while (u < u1) {
+        const int nb = KSB == 1 ? 1 : blocks_of(ks);
+        const int jb = KSB == 1 ? 0 : (set - i) & (kSets - 1);  // the set's block of this slab, if it has one
+        const uint32_t slab = p.c_addr[slot], bar = c_empty + 8 * slot;
+        if (!mbar_wait(c_full + 8 * slot, c_phase)) { timed_out = true; return -1; }
+        const bool mine = jb < nb;
+        if (mine) {
+          codes.load(slab + slab_off, jb, g, r, half, x);
+          const uint32_t scw = ring32(slab + scale_off + jb * 128);
+          s2 = half ? prmt<0x3232>(scw, 0u) : prmt<0x1010>(scw, 0u);
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar);
+        const int block = KSB == 1 ? u - u0 : i + jb;
+        if constexpr (KSB == 1) {
+          u += kSets;
+          slot += kSets;
+          if (slot >= p.code_slots) { slot -= p.code_slots; c_phase ^= 1; }
+        } else {
+          ++u;
+          i += nb;
+          if (++ks == p.k_slabs) ks = 0;
+          if (++slot == p.code_slots) { slot = 0; c_phase ^= 1; }
+        }
+        if (mine) return block;
+      }
+      return -1;
+    };
+    // A block's stores to tensor memory are awaited and handed over while the lookups of the next
+    // one are in flight, whose codes were fetched between the two halves of this one.
+    auto hand_over = [&](int s) {
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(full + 8 * s);
+    };
+    RowCodes<BITS> codes;
+    uint32_t s2 = 0;
+    int block = fetch(codes, s2), stored = -1;
+    while (block >= 0) {
+      const int s = block & (S - 1);
+      uint32_t v[16];
+      codes.template decode<0, FP16, WIDE>(lane_base, s2, v, 0);
+      codes.template decode<1, FP16, WIDE>(lane_base, s2, v, 8);
+      if (stored >= 0) hand_over(stored);
+      if (!mbar_wait(empty + 8 * s, ((block >> p.stages_log2) & 1) ^ 1)) { timed_out = true; break; }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      tmem_store16(a_lane + 32 * s, v);
+      codes.template decode<2, FP16, WIDE>(lane_base, s2, v, 0);
+      codes.template decode<3, FP16, WIDE>(lane_base, s2, v, 8);
+      block = fetch(codes, s2);
+      tmem_store16(a_lane + 32 * s + 16, v);
+      stored = s;
+    }
+    if (stored >= 0 && !timed_out) hand_over(stored);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    last_epilogue(set);
   }
   if (timed_out && lane == 0) atomicOr(p.status, kTcStatusTimeout);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == 1) {
+  if (warp == kTcMmaWarp) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(p.tmem_cols) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)kTcTmemColumns) : "memory");
   }
 }
 
@@ -448,36 +632,41 @@ int encode_fn(EncodeTiledFn* out) {
 }
 
 inline uint32_t round_up(uint32_t v, uint32_t a) { return (v + a - 1) / a * a; }
-inline bool two_per_sm(int m_pad) { return m_pad <= 64; }
 
-// Shared memory: barriers, the table, then the stage buffers (1024-byte aligned for the
-// swizzled tiles).  Returns the dynamic size, or 0 if `stages` do not fit in `limit`.
+// Shared memory: barriers, the table (a wide one at a multiple of 64 KB of the shared window, with
+// buffers on both sides of it), the x stages (1024-byte aligned for the swizzle), the code
+// ring: as many slots as fit, up to sixteen (68 KB of 4-bit codes in flight per SM; four are
+// the least, see the dequantising warps).  Returns the dynamic size, or 0 if nothing fits.
 template <int BITS>
-size_t plan_tc_smem(uint32_t base, uint32_t limit, int stages, TcParams& p) {
+size_t plan_tc_smem(uint32_t base, uint32_t limit, TcParams& p) {
   using L = Layout<BITS>;
-  using T = Table<BITS>;
-  uint32_t cursor = round_up(base, 128);
+  using T = Table<BITS, kTcWideTable<BITS>>;
+  const uint32_t end = base + limit;
+  uint32_t low = round_up(base, 128);  // next free address below the table
   p.smem_base = base;
-  p.bar_addr = cursor;
-  p.tmem_slot_addr = cursor + 8 * (3 * kTcMaxStages + 1);  // then the four code-ring barriers
-  cursor += 256;
-  p.table_addr = cursor;
-  cursor += T::kBytes;
-  p.stages = stages;
-  const uint32_t b_bytes = (uint32_t)p.m_pad * 128;
-  cursor = round_up(cursor, 1024);
-  for (int s = 0; s < stages; ++s) { p.b_addr[s] = cursor; cursor += b_bytes; }
-  for (int s = 0; s < stages; ++s) { p.a_addr[s] = cursor; cursor += 16384; }
-  if (L::KSB == 1) {
-    for (int s = 0; s < stages; ++s) { p.c_addr[s] = cursor; cursor += round_up(2 * L::kSlabBytes, 128); }
-  } else {
-    for (int c = 0; c < 2; ++c) { p.cc_addr[c] = cursor; cursor += round_up(2 * L::kSlabBytes, 128); }
-  }
-  return (cursor - base <= limit) ? cursor - base : 0;
+  p.bar_addr = low;
+  low += 512;
+  p.table_addr = round_up(low, kTcWideTable<BITS> ? 65536 : 128);
+  uint32_t high = p.table_addr + T::kBytes, used = high;
+  if (high > end) return 0;
+  auto take = [&](uint32_t bytes, uint32_t align) -> uint32_t {
+    uint32_t a = round_up(low, align);
+    if (a + bytes <= p.table_addr) { low = a + bytes; return a; }
+    a = round_up(high, align);
+    if (a + bytes > end) return 0;
+    high = used = a + bytes;
+    return a;
+  };
+  for (int s = 0; s < (1 << p.stages_log2); ++s)
+    if ((p.b_addr[s] = take((uint32_t)p.n_tile * 128, 1024)) == 0) return 0;
+  int slots = 0;
+  while (slots < kTcMaxCodeSlots && (p.c_addr[slots] = take(round_up(2 * L::kSlabBytes, 128), 128)) != 0) ++slots;
+  p.code_slots = slots & ~3;
+  return p.code_slots >= 4 ? used - base : 0;
 }
 
 template <int BITS, bool FP16>
-int launch_tc(TcParams p, const void* lut_host, const CUtensorMap& map, int tiles, cudaStream_t stream) {
+int launch_tc(TcParams p, const void* lut_host, const CUtensorMap& map, int grid, bool pdl, cudaStream_t stream) {
   InlineLut<BITS> inl;
   if (lut_host != nullptr) {
     memcpy(inl.w, lut_host, sizeof(inl.w));
@@ -489,11 +678,7 @@ int launch_tc(TcParams p, const void* lut_host, const CUtensorMap& map, int tile
   if (int st = dynamic_smem_base(&base)) return st;
   DeviceInfo di;
   if (int st = device_info(&di)) return st;
-  size_t smem = 0;
-  // small batches: two CTAs per SM (twice the warps to hide the latencies of the per-block
-  // hand-offs), each within half the shared memory; tensor memory holds both accumulators
-  const uint32_t limit = two_per_sm(p.m_pad) ? ((uint32_t)di.max_smem_optin + 1024) / 2 - 1024 : (uint32_t)di.max_smem_optin;
-  for (int s = kTcMaxStages; s >= 1 && smem == 0; --s) smem = plan_tc_smem<BITS>(base, limit, s, p);
+  const size_t smem = plan_tc_smem<BITS>(base, (uint32_t)di.max_smem_optin, p);
   FDK_CHECK_ARG(smem != 0, FDK_ERR_CUDA, "no shared-memory plan fits %d bytes", di.max_smem_optin);
   auto kernel = gemm_lut_tc_kernel<BITS, FP16>;
   static size_t configured[64] = {};
@@ -503,8 +688,17 @@ int launch_tc(TcParams p, const void* lut_host, const CUtensorMap& map, int tile
     FDK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     configured[dev & 63] = smem;
   }
-  kernel<<<tiles, kTcThreads, smem, stream>>>(p, inl, map);
-  FDK_CUDA(cudaGetLastError());
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(kTcThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  FDK_CUDA(cudaLaunchKernelEx(&cfg, kernel, p, inl, map));
   return FDK_OK;
 }
 
@@ -512,67 +706,65 @@ int launch_tc(TcParams p, const void* lut_host, const CUtensorMap& map, int tile
 
 // Batches above 16 rows.  Called by fdk_linear_lut.
 int gemm_lut_tc(const void* x, const void* tiled, const void* lut, const void* lut_host, void* out, int m, int n,
-                int k, int bits, bool fp16, void* workspace, size_t workspace_bytes, int sm_count, cudaStream_t stream) {
+                int k, int bits, bool fp16, void* workspace, size_t workspace_bytes, int sm_count, bool pdl,
+                cudaStream_t stream) {
   EncodeTiledFn encode = nullptr;
   if (int st = encode_fn(&encode)) return st;
   const TiledDims d = tiled_dims(n, k, bits);
-  const int tiles = (n + kTcTileRows - 1) / kTcTileRows;
-  const int k_blocks = k / kBlock;
-  // few tiles: several CTAs share a tile, each with its own range of 64-column blocks, so that
-  // the whole GPU is busy; all of them must be resident at once (the owner waits for the others)
-  const int m_pad_max = ((m < 256 ? m : 256) + 15) / 16 * 16;
-  const int resident = sm_count * (two_per_sm(m_pad_max) ? 2 : 1);
-  int splits = 1;
-  if (tiles * 2 <= resident) {
-    splits = resident / tiles;
-    if (splits > kTcMaxSplits) splits = kTcMaxSplits;
-    if (splits > k_blocks / 4) splits = k_blocks / 4;
-    if (splits < 1) splits = 1;
+  TcParams p{};
+  p.tiled = (const uint8_t*)tiled;
+  p.lut = lut;
+  p.out = (uint16_t*)out;
+  p.status = (int*)workspace + kStatusWord;
+  p.m = m;
+  p.n = n;
+  p.m_tiles = (m + kTcMaxBatch - 1) / kTcMaxBatch;
+  p.n_tile = (int)round_up((uint32_t)((m + p.m_tiles - 1) / p.m_tiles), 16);
+  p.row_tiles = d.row_tiles;
+  p.k_blocks = k / kBlock;
+  p.k_slabs = d.k_slabs;
+  const long long tiles = (long long)((n + kTcTileRows - 1) / kTcTileRows) * p.m_tiles, units = tiles * d.k_slabs;
+  FDK_CHECK_ARG(units < (1ll << 31), FDK_ERR_SHAPE, "m=%d, n=%d, k=%d: too many tiles", m, n, k);
+  p.tiles = (int)tiles;
+  // up to 128 batch rows eight A stages and two accumulators fit tensor memory, up to 192 four and two
+  p.stages_log2 = p.n_tile <= 128 ? 3 : 2;
+  p.acc_slots = p.n_tile <= 192 ? 2 : 1;
+  p.flags = (int*)((uint8_t*)workspace + kTcFlagsOffset);
+  p.partial = (float*)((uint8_t*)workspace + kTcPartialOffset);
+  // One CTA per SM.  Ranges cut tiles where the workspace has room for every CTA's partial sums.
+  // Where a tile is shared by many CTAs its owner reads all their sums (about 10 cycles per CTA and
+  // batch row), which has to stay below what the CTAs save (max(2 n_tile, 250) cycles per block):
+  // the total  units t / G + G / tiles 10 n_tile  is least at the G below.
+  int grid = sm_count;
+  const size_t slot_bytes = (size_t)p.n_tile * kTcTileRows * sizeof(float);
+  const size_t room = workspace_bytes > kTcPartialOffset ? (workspace_bytes - kTcPartialOffset) / slot_bytes : 0;
+  if (tiles < grid) {
+    const double block = 2.0 * p.n_tile > 250.0 ? 2.0 * p.n_tile : 250.0;
+    const double best = std::sqrt((double)p.k_blocks * tiles * block * tiles / (10.0 * p.n_tile));
+    const long long four = (long long)p.k_blocks * tiles / 4;  // at least four blocks each
+    if (best < grid) grid = (int)best;
+    if (four < grid) grid = (int)four;
+    if (units < grid) grid = (int)units;
+    if (grid < tiles) grid = (int)tiles;
   }
-  // the parked partial tiles (128 rows x m_pad columns of fp32 each) must fit the workspace
-  const size_t partial_room = workspace_bytes > kTcPartialOffset ? workspace_bytes - kTcPartialOffset : 0;
-  while (splits > 1 && ((size_t)tiles * (splits - 1) * 128 * m_pad_max * sizeof(float) > partial_room || tiles > 2048)) --splits;
-  for (int m0 = 0; m0 < m; m0 += 256) {
-    const int mc = (m - m0) < 256 ? (m - m0) : 256;
-    TcParams p{};
-    p.tiled = (const uint8_t*)tiled;
-    p.lut = lut;
-    p.out = (uint16_t*)out + (size_t)m0 * n;
-    p.status = (int*)workspace + kStatusWord;
-    p.m = mc;
-    p.m_pad = (mc + 15) / 16 * 16;
-    p.n = n;
-    p.k = k;
-    p.row_tiles = d.row_tiles;
-    p.k_blocks = k_blocks;
-    p.k_slabs = d.k_slabs;
-    p.splits = splits;
-    p.flags = (int*)((uint8_t*)workspace + kTcFlagsOffset);
-    p.uses = (int*)((uint8_t*)workspace + kTcUsesOffset);
-    p.partial = (float*)((uint8_t*)workspace + kTcPartialOffset);
-    uint32_t cols = 32;
-    while ((int)cols < p.m_pad) cols *= 2;
-    p.tmem_cols = cols;
-    CUtensorMap map;
-    const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)mc};
-    const cuuint64_t strides[1] = {(cuuint64_t)k * 2};
-    const cuuint32_t box[2] = {64, (cuuint32_t)p.m_pad};
-    const cuuint32_t elem[2] = {1, 1};
-    CUresult r = encode(&map, fp16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void*)((const uint16_t*)x + (size_t)m0 * k), dims,
-                        strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                        CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    FDK_CHECK_ARG(r == CUDA_SUCCESS, FDK_ERR_CUDA, "cuTensorMapEncodeTiled failed with %d", (int)r);
-    int st;
-    switch (bits) {
-      case 1: st = fp16 ? launch_tc<1, true>(p, lut_host, map, tiles * splits, stream) : launch_tc<1, false>(p, lut_host, map, tiles * splits, stream); break;
-      case 2: st = fp16 ? launch_tc<2, true>(p, lut_host, map, tiles * splits, stream) : launch_tc<2, false>(p, lut_host, map, tiles * splits, stream); break;
-      case 3: st = fp16 ? launch_tc<3, true>(p, lut_host, map, tiles * splits, stream) : launch_tc<3, false>(p, lut_host, map, tiles * splits, stream); break;
-      case 4: st = fp16 ? launch_tc<4, true>(p, lut_host, map, tiles * splits, stream) : launch_tc<4, false>(p, lut_host, map, tiles * splits, stream); break;
-      default: st = fp16 ? launch_tc<8, true>(p, lut_host, map, tiles * splits, stream) : launch_tc<8, false>(p, lut_host, map, tiles * splits, stream); break;
-    }
-    if (st) return st;
+  p.split = room >= (size_t)grid && grid * kTcFlagsPerRank * sizeof(int) <= kTcPartialOffset - kTcFlagsOffset;
+  if (!p.split && tiles < grid) grid = (int)tiles;
+  CUtensorMap map;
+  const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)m};
+  const cuuint64_t strides[1] = {(cuuint64_t)k * 2};
+  const cuuint32_t box[2] = {64, (cuuint32_t)p.n_tile};
+  const cuuint32_t elem[2] = {1, 1};
+  CUresult r = encode(&map, fp16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void*)x, dims,
+                      strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                      CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  FDK_CHECK_ARG(r == CUDA_SUCCESS, FDK_ERR_CUDA, "cuTensorMapEncodeTiled failed with %d", (int)r);
+  switch (bits) {
+    case 1: return fp16 ? launch_tc<1, true>(p, lut_host, map, grid, pdl, stream) : launch_tc<1, false>(p, lut_host, map, grid, pdl, stream);
+    case 2: return fp16 ? launch_tc<2, true>(p, lut_host, map, grid, pdl, stream) : launch_tc<2, false>(p, lut_host, map, grid, pdl, stream);
+    case 3: return fp16 ? launch_tc<3, true>(p, lut_host, map, grid, pdl, stream) : launch_tc<3, false>(p, lut_host, map, grid, pdl, stream);
+    case 4: return fp16 ? launch_tc<4, true>(p, lut_host, map, grid, pdl, stream) : launch_tc<4, false>(p, lut_host, map, grid, pdl, stream);
+    default: return fp16 ? launch_tc<8, true>(p, lut_host, map, grid, pdl, stream) : launch_tc<8, false>(p, lut_host, map, grid, pdl, stream);
   }
-  return FDK_OK;
 }
 
 }  // namespace fdk

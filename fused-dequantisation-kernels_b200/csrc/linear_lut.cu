@@ -173,8 +173,7 @@ static int linear_lut_impl(const void* x, const void* tiled, const void* lut, co
   // at 8192^2 against 29-30 us for the tensor-core kernel and 26 us for bf16 cuBLAS)
   if (fu == nullptr && ex == nullptr && !(flags & FDK_FLAG_SILU_PAIRS) && m > 16) {
     return gemm_lut_tc(x, tiled, lut, lut_host, out, m, n, k, bits, dtype == FDK_DTYPE_F16, workspace, workspace_bytes,
-                       di.sm_count,
-                       (cudaStream_t)stream);
+                       di.sm_count, (flags & FDK_FLAG_PDL) != 0, (cudaStream_t)stream);
   }
   for (int m0 = 0; m0 < m; m0 += 16) {
     p.m = (m - m0) < 16 ? (m - m0) : 16;

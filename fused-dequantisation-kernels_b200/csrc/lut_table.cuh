@@ -236,20 +236,20 @@ __device__ __forceinline__ int ld_relaxed_s32(const int* p) {
 // ---- workspace layout (bytes) -----------------------------------------------------------------
 //   [0, 16 KB)            use counts of split row tiles (4095 ints) + the status word
 //   [16 KB, kGemvEnd)     tagged partial sums of the GEMV kernel, 8 KB per SM, room for 160 SMs
-//   then 8 KB of flags and 8 KB of tile use counts of the tensor-core GEMM
-//   then its fp32 partial tiles: up to 148 tiles of 128 rows x 256 batch columns
+//   then 40 KB of flags of the tensor-core GEMM (64 per CTA; zero between launches)
+//   then its fp32 partial tiles: one of 128 rows x up to 256 batch columns per CTA, room for 148
 constexpr size_t kCounterBytes = 16384;
 constexpr int kStatusWord = 4095;
 constexpr size_t kGemvEnd = kCounterBytes + (size_t)160 * 1024 * sizeof(uint2);
 constexpr size_t kTcFlagsOffset = kGemvEnd;
-constexpr size_t kTcUsesOffset = kGemvEnd + 8192;
-constexpr size_t kTcPartialOffset = kGemvEnd + 16384;
+constexpr size_t kTcPartialOffset = kTcFlagsOffset + (size_t)160 * 64 * sizeof(int);
 constexpr size_t kTcPartialTileBytes = (size_t)128 * 256 * sizeof(float);
 constexpr size_t kWorkspaceBytes = kTcPartialOffset + 148 * kTcPartialTileBytes;
 
-// Tensor-core GEMM for batches above 8 rows (gemm_lut_tc.cu).
+// Tensor-core GEMM for batches above 16 rows (gemm_lut_tc.cu).
 int gemm_lut_tc(const void* x, const void* tiled, const void* lut, const void* lut_host, void* out, int m, int n,
-                int k, int bits, bool fp16, void* workspace, size_t workspace_bytes, int sm_count, cudaStream_t stream);
+                int k, int bits, bool fp16, void* workspace, size_t workspace_bytes, int sm_count, bool pdl,
+                cudaStream_t stream);
 
 // The dynamic shared memory address seen by kernels without static shared memory, asked of
 // the device once (linear_lut.cu).

@@ -1,0 +1,66 @@
+"""The tensor-core GEMM where its work split can go wrong: batch sizes around the tile and stage limits, tiles
+cut by many ranges, short last slabs, several shapes in turn through one workspace."""
+
+import ctypes
+
+import pytest
+import torch
+
+from fdk import models, native
+
+pytestmark = pytest.mark.gpu
+
+
+def problem(m, n, k, bits, dtype):
+    gen = torch.Generator(device="cuda").manual_seed(m + n + k + bits)
+    w = (torch.randn((n, k), generator=gen, device="cuda") * k**-0.5).to(dtype)
+    layer = models.QuantisedLinear.create(w, models.QuantisationConfig(bits, 64))
+    x = torch.randn((m, k), generator=gen, device="cuda").to(dtype)
+    dense = native.dequantise(layer.weight_data, layer.lut, layer.scale, bits)
+    return layer, x, x.double() @ dense.double().t()
+
+
+def check(y, want, dtype):
+    # fp32 sums of exact products, one rounding of the result: half a unit in the last place, uniform
+    # over a binade, is 2^-9 / sqrt(3) relative at most (bf16; 2^-12 / sqrt(3) fp16), plus the sums' own 1e-5
+    unit = 2.0**-9 if dtype == torch.bfloat16 else 2.0**-12
+    assert ((y.double() - want).norm() / want.norm()).item() < unit + 1e-5
+    assert bool(y.isfinite().all())
+
+
+@pytest.mark.parametrize("bits", [1, 2, 3, 4, 8])
+@pytest.mark.parametrize("m", [17, 64, 65, 128, 129, 192, 193, 256, 257, 700])
+def test_batch_limits(m, bits):
+    dtype = torch.float16 if m % 2 else torch.bfloat16
+    n, k = (1100, 64 * 37) if m < 300 else (333, 64 * 9)  # ragged last tile, short last slab
+    layer, x, want = problem(m, n, k, bits, dtype)
+    check(layer(x), want, dtype)
+    assert native.device_status() == 0
+
+
+def test_many_ranges_and_shapes_share_a_workspace():
+    """Few tiles over long rows: most CTAs hold the middle of a tile.  Every launch leaves the hand-over flags
+    clear for the next one, whatever its shape, and results repeat bit for bit."""
+    shapes = [(40, 64, 64 * 150, 4), (250, 130, 64 * 260, 8), (24, 5120, 3072, 4), (200, 1024, 64 * 129, 2), (600, 640, 64 * 33, 3)]
+    cases = [problem(*s, torch.bfloat16) for s in shapes]
+    first = [layer(x) for layer, x, _ in cases]
+    for layer_x, y in list(zip(cases, first)) * 3:
+        layer, x, want = layer_x
+        again = layer(x)
+        assert torch.equal(again, y)
+        check(again, want, torch.bfloat16)
+    assert native.device_status() == 0
+
+
+@pytest.mark.parametrize("m,n,k", [(40, 300, 640), (300, 128, 192)])
+def test_without_room_for_partial_sums(m, n, k):
+    """The scratch built into the library holds none: tiles are not cut."""
+    layer, x, want = problem(m, n, k, 4, torch.bfloat16)
+    out = torch.full((m, n), float("nan"), device="cuda", dtype=torch.bfloat16)
+    status = native.lib().fdk_linear_lut_static(
+        x.data_ptr(), layer.tiled().data_ptr(), layer.lut.data_ptr(), layer.lut_bytes(), out.data_ptr(), m, n, k, 4,
+        native.DTYPE_BF16, 0, native._stream())
+    assert status == 0
+    check(out, want, torch.bfloat16)
+    word = ctypes.c_int(0)
+    assert native.lib().fdk_static_status(ctypes.byref(word)) == 0 and word.value == 0
