@@ -243,6 +243,60 @@ __global__ void rope_append_kernel(const uint16_t* __restrict__ qkv, const long 
   dst[i + 64] = o1;
 }
 
+// Rotary embedding of a whole prompt, and its keys and values into the caches: qkv [batch * T, heads * 128]
+// (q and k heads in the paired order, see above), table [T][64] of {bf16 cos, bf16 sin} -> q
+// [batch, q_heads, T, 128] and positions 0 .. T - 1 of the caches.  The values of rope_append_kernel.
+// Bound by HBM (every value read and written once); a thread takes eight of the 64 pairs of a
+// head, two 16-byte vectors each way, neighbouring threads neighbouring vectors.  1000 tokens of 24 + 2 x
+// 8 heads: replaces about 25 framework launches a layer.
+__global__ void rope_prefill_kernel(const uint16_t* __restrict__ qkv, const uint32_t* __restrict__ table,
+                                    uint16_t* __restrict__ q_out, uint16_t* __restrict__ k_cache,
+                                    uint16_t* __restrict__ v_cache, int t_count, int q_heads, int kv_heads, int max_len,
+                                    long long total) {
+  pdl_prologue();
+  const int heads_total = q_heads + 2 * kv_heads;
+  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x) {
+    const int i = (int)(idx & 7) * 8;  // pairs i .. i + 7
+    const long long rest = idx >> 3;
+    const int head = (int)(rest % heads_total);
+    const long long row = rest / heads_total;
+    const int t = (int)(row % t_count);
+    const long long b = row / t_count;
+    const uint16_t* src = qkv + (row * heads_total + head) * 128;
+    if (head >= q_heads + kv_heads) {
+      uint16_t* dst = v_cache + ((b * kv_heads + (head - q_heads - kv_heads)) * max_len + t) * 128;
+      *reinterpret_cast<uint4*>(dst + i) = *reinterpret_cast<const uint4*>(src + i);
+      *reinterpret_cast<uint4*>(dst + i + 64) = *reinterpret_cast<const uint4*>(src + i + 64);
+      continue;
+    }
+    const int at = i < 32 ? i : i + 32;
+    const uint4 v0 = *reinterpret_cast<const uint4*>(src + at), v1 = *reinterpret_cast<const uint4*>(src + at + 32);
+    const uint4* tab = reinterpret_cast<const uint4*>(table + (size_t)t * 64 + i);
+    const uint4 t0 = __ldg(tab), t1 = __ldg(tab + 1);
+    const uint32_t a[4] = {v0.x, v0.y, v0.z, v0.w}, c[4] = {v1.x, v1.y, v1.z, v1.w};
+    const uint32_t cs[8] = {t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w};
+    uint32_t lo[4], hi[4];
+    auto r = [](float v) { return to_float<false>(from_float<false>(v)); };
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      uint32_t out0[2], out1[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const float x0 = e ? pair_hi<false>(a[j]) : pair_lo<false>(a[j]), x1 = e ? pair_hi<false>(c[j]) : pair_lo<false>(c[j]);
+        const float co = pair_lo<false>(cs[2 * j + e]), si = pair_hi<false>(cs[2 * j + e]);
+        out0[e] = from_float<false>(r(x0 * co) + r(-x1 * si));
+        out1[e] = from_float<false>(r(x1 * co) + r(x0 * si));
+      }
+      lo[j] = out0[0] | (out0[1] << 16);
+      hi[j] = out1[0] | (out1[1] << 16);
+    }
+    uint16_t* dst = head < q_heads ? q_out + ((b * q_heads + head) * t_count + t) * 128
+                                   : k_cache + ((b * kv_heads + (head - q_heads)) * max_len + t) * 128;
+    *reinterpret_cast<uint4*>(dst + i) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    *reinterpret_cast<uint4*>(dst + i + 64) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+  }
+}
+
 // table[i] = {bf16 cos, bf16 sin} of angle pos * theta^(-2 i / 128), i = 0 .. 63: what every
 // rotary embedding of one decode step needs, computed once per step (the values of
 // rope_append_kernel above).
@@ -483,6 +537,21 @@ extern "C" int fdk_rope_append_paired(const void* qkv, const void* pos, void* q_
                                       int rows, int q_heads, int kv_heads, int head_dim, int max_len, float theta,
                                       void* stream) {
   return rope_append_impl(qkv, pos, q_out, k_cache, v_cache, rows, q_heads, kv_heads, head_dim, max_len, theta, 1, stream);
+}
+
+extern "C" int fdk_rope_prefill_paired(const void* qkv, const void* table, void* q_out, void* k_cache, void* v_cache, int batch,
+                                       int tokens, int q_heads, int kv_heads, int head_dim, int max_len, void* stream) {
+  FDK_CHECK_ARG(qkv && table && q_out && k_cache && v_cache, FDK_ERR_BAD_ARG, "null pointer");
+  FDK_CHECK_ARG(head_dim == 128, FDK_ERR_SHAPE, "head_dim=%d: only 128 is supported", head_dim);
+  FDK_CHECK_ARG(batch > 0 && tokens > 0 && q_heads > 0 && kv_heads > 0 && tokens <= max_len, FDK_ERR_BAD_ARG,
+                "batch=%d, tokens=%d, heads=%d + %d, max_len=%d", batch, tokens, q_heads, kv_heads, max_len);
+  FDK_CHECK_ARG((((uintptr_t)qkv | (uintptr_t)table | (uintptr_t)q_out | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15) == 0,
+                FDK_ERR_ALIGN, "pointers must be 16-byte aligned");
+  const long long total = (long long)batch * tokens * (q_heads + 2 * kv_heads) * 8;
+  const long long blocks = (total + 255) / 256;
+  return launch_pdl(rope_prefill_kernel, dim3((unsigned)(blocks < 148 * 16 ? blocks : 148 * 16)), dim3(256), 0,
+                    (cudaStream_t)stream, (const uint16_t*)qkv, (const uint32_t*)table, (uint16_t*)q_out, (uint16_t*)k_cache,
+                    (uint16_t*)v_cache, tokens, q_heads, kv_heads, max_len, total);
 }
 
 extern "C" int fdk_rope_table(const void* pos, void* table, float theta, void* stream) {

@@ -356,8 +356,8 @@ class LlamaDecoder(nn.Module):
         position [batch, vocab]; fills the KV caches and leaves the position at T.  One pass over
         the whole prompt, as the reference's Generator does with transformers' model
         (src/fdk/models.py:241-243): the projections run the fused kernels on [batch * T, K]
-        (the tensor-core kernel from 17 rows on), the norms the RMSNorm kernel; rotary embedding and
-        causal attention over the prompt are torch ops (this path runs once per sequence)."""
+        (the tensor-core kernel from 17 rows on), the norms the RMSNorm kernel, the rotary embedding and the
+        cache append a kernel of their own; causal attention over the prompt is a torch op."""
         dims, eps = self.dims, self.dims.rms_norm_eps
         batch, t = ids.shape
         assert batch == self.batch and t <= self.max_len, f"prompt {tuple(ids.shape)} for caches of {self.batch} x {self.max_len}"
@@ -365,26 +365,17 @@ class LlamaDecoder(nn.Module):
         rows = batch * t
         hidden = self.embed.weight[ids.reshape(-1)].contiguous()  # [rows, hidden]
         normed = torch.empty_like(hidden)
-        unpair = torch.argsort(torch.tensor(ROPE_ROW_ORDER, device=dev))  # paired row order -> dimensions 0 .. 127
         inv_freq = 1.0 / (dims.rope_theta ** (torch.arange(0, 128, 2, dtype=torch.float32, device=dev) / 128))
         angles = torch.arange(t, dtype=torch.float32, device=dev)[:, None] * inv_freq[None, :]
-        emb = torch.cat((angles, angles), dim=-1)
-        cos, sin = emb.cos().bfloat16()[None, :, None, :], emb.sin().bfloat16()[None, :, None, :]  # [1, T, 1, 128]
-
-        def rotate(x):  # [batch, T, heads, 128], transformers' rotate-half form
-            return x * cos + torch.cat((-x[..., 64:], x[..., :64]), dim=-1) * sin
+        table = torch.stack((angles.cos(), angles.sin()), dim=-1).bfloat16()  # [T, 64, 2]
+        q = torch.empty((batch, self.q_heads, t, 128), device=dev, dtype=torch.bfloat16)
 
         delta = None
         for i, layer in enumerate(self.layers):
             native.rmsnorm(hidden, delta, layer.input_norm, normed, eps)
-            qkv = layer.qkv(normed).view(batch, t, self.q_heads + 2 * self.kv_heads, 128)
-            q = rotate(qkv[:, :, : self.q_heads][..., unpair])
-            k = rotate(qkv[:, :, self.q_heads: self.q_heads + self.kv_heads][..., unpair])
-            v = qkv[:, :, self.q_heads + self.kv_heads:]
-            self.k_cache[i][:, :, :t] = k.transpose(1, 2)
-            self.v_cache[i][:, :, :t] = v.transpose(1, 2)
+            native.rope_prefill(layer.qkv(normed), table, q, self.k_cache[i], self.v_cache[i])
             attn = nn.functional.scaled_dot_product_attention(
-                q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2), is_causal=True, enable_gqa=True
+                q, self.k_cache[i][:, :, :t], self.v_cache[i][:, :, :t], is_causal=True, enable_gqa=True
             ).transpose(1, 2).reshape(rows, self.q_heads * 128).contiguous()
             delta = layer.o(attn)
             self.tp.all_reduce(delta)

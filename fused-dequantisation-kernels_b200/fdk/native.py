@@ -122,6 +122,7 @@ _SIGNATURES = {
     "fdk_rmsnorm": (ctypes.c_int, [ctypes.c_void_p] * 4 + [ctypes.c_int] * 2 + [ctypes.c_float, ctypes.c_void_p]),
     "fdk_rope_append": (ctypes.c_int, [ctypes.c_void_p] * 5 + [ctypes.c_int] * 5 + [ctypes.c_float, ctypes.c_void_p]),
     "fdk_rope_append_paired": (ctypes.c_int, [ctypes.c_void_p] * 5 + [ctypes.c_int] * 5 + [ctypes.c_float, ctypes.c_void_p]),
+    "fdk_rope_prefill_paired": (ctypes.c_int, [ctypes.c_void_p] * 5 + [ctypes.c_int] * 6 + [ctypes.c_void_p]),
     "fdk_silu_mul": (ctypes.c_int, [ctypes.c_void_p] * 2 + [ctypes.c_int] * 3 + [ctypes.c_void_p]),
     "fdk_decode_attention_scratch": (ctypes.c_int, [ctypes.c_int] * 4 + [ctypes.POINTER(ctypes.c_size_t)] * 2),
     "fdk_decode_attention": (ctypes.c_int, [ctypes.c_void_p] * 7 + [ctypes.c_int] * 6 + [ctypes.c_void_p]),
@@ -562,6 +563,25 @@ def rope_append(
             (lib().fdk_rope_append_paired if paired else lib().fdk_rope_append)(
                 qkv.data_ptr(), pos.data_ptr(), q_out.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),
                 qkv.shape[0], q_heads, kv_heads, 128, k_cache.shape[2], theta, _stream(),
+            )
+        )
+
+
+def rope_prefill(qkv: Tensor, table: Tensor, q_out: Tensor, k_cache: Tensor, v_cache: Tensor) -> None:
+    """Rotary embedding of a prompt's fused q|k|v projections [batch * T, heads * 128] (q and k heads in the
+    paired row order): q_out [batch, q_heads, T, 128], k and v to positions 0 .. T - 1 of the caches
+    [batch, kv_heads, max_len, 128].  table [T, 64, 2]: cosines and sines."""
+    _require_cuda(qkv, table, q_out, k_cache, v_cache)
+    batch, q_heads, tokens, _ = q_out.shape
+    kv_heads, max_len = k_cache.shape[1:3]
+    assert all(t.is_contiguous() and t.dtype == torch.bfloat16 for t in (qkv, table, q_out, k_cache, v_cache))
+    assert qkv.shape == (batch * tokens, (q_heads + 2 * kv_heads) * 128) and table.shape == (tokens, 64, 2)
+    assert k_cache.shape == v_cache.shape == (batch, kv_heads, max_len, 128)
+    with torch.cuda.device(qkv.device):
+        check(
+            lib().fdk_rope_prefill_paired(
+                qkv.data_ptr(), table.data_ptr(), q_out.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),
+                batch, tokens, q_heads, kv_heads, 128, max_len, _stream(),
             )
         )
 
