@@ -84,23 +84,21 @@ class QuantisedLinear(nn.Module):
 
     def tiled(self) -> Tensor:
         """The kernels' tiled copy of (weight_data, scale); rebuilt when they change or move."""
-        key = (
-            self.weight_data.data_ptr(), self.scale.data_ptr(),
-            self.weight_data._version, self.scale._version, str(self.weight_data.device),
-        )
+        weight, scale = self.weight_data, self.scale  # (each a lookup through the module's dictionaries)
+        key = (weight.data_ptr(), scale.data_ptr(), weight._version, scale._version, weight.device)
         if self._tiled is None or self._tiled_key != key:
             self._tiled = native.repack(
-                self.weight_data.data, self.scale.data, self.out_features, self.in_features,
-                self.bits, self.block_size,
+                weight.data, scale.data, self.out_features, self.in_features, self.bits, self.block_size,
             )
             self._tiled_key = key
         return self._tiled
 
     def lut_bytes(self) -> bytes:
         """Host copy of the table (made once): it travels with the kernel's launch parameters."""
-        key = (self.lut.data_ptr(), self.lut._version)
-        if getattr(self, "_lut_host_key", None) != key:
-            self._lut_host = native.host_lut(self.lut)
+        lut = self.lut
+        key = (lut.data_ptr(), lut._version)
+        if self.__dict__.get("_lut_host_key") != key:
+            self._lut_host = native.host_lut(lut)
             self._lut_host_key = key
         return self._lut_host
 
@@ -111,9 +109,10 @@ class QuantisedLinear(nn.Module):
             return kernels.mm_lut_ref(x, self.weight_data, self.lut, self.scale)
         assert self.kernel in ("triton", "marlin", "marlin-lut")
         out = torch.empty((x.shape[0], self.out_features), device=x.device, dtype=x.dtype)
-        assert x.dtype == self.lut.dtype == self.scale.dtype
+        lut = self.lut
+        assert x.dtype == lut.dtype == self.scale.dtype
         native.linear_lut(
-            x.contiguous(), self.tiled(), self.lut, out, self.out_features, self.in_features, self.bits,
+            x.contiguous(), self.tiled(), lut, out, self.out_features, self.in_features, kernels.bits_of_lut(lut),
             pdl=True, lut_bytes=self.lut_bytes(),
         )
         return out

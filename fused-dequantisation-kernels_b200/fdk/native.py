@@ -10,6 +10,7 @@ from __future__ import annotations
 import ctypes
 import os
 import weakref
+from contextlib import nullcontext
 from pathlib import Path
 
 import torch
@@ -187,7 +188,16 @@ def dtype_code(dtype: torch.dtype) -> int:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current device's current stream (the handle alone: a stream object costs over a microsecond)."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+
+
+_HERE = nullcontext()
+
+
+def _on(device: torch.device):
+    """`torch.cuda.device(device)`, at no cost where that is the current device already."""
+    return _HERE if device.index == torch.cuda.current_device() else torch.cuda.device(device)
 
 
 def _require_cuda(*tensors: Tensor) -> None:
@@ -226,7 +236,7 @@ def quantise(weight: Tensor, bits: int, block_size: int, lut: Tensor, scale: Ten
     table = torch.empty((8, 1) if bits == 3 else (256, 8 // bits), dtype=dt, device=dev)
     out_scale = torch.empty((n, k // block_size), dtype=dt, device=dev) if scale is None else scale
     lut = lut.detach().contiguous()
-    with torch.cuda.device(dev):
+    with _on(dev):
         check(
             lib().fdk_quantise(
                 weight.data_ptr(), n, k, bits, block_size, dtype_code(dt), lut.data_ptr(), lut.shape[0],
@@ -242,7 +252,7 @@ def repack(codes: Tensor, scale: Tensor, n: int, k: int, bits: int, block_size: 
     _require_cuda(codes, scale)
     assert codes.dtype == torch.uint8 and codes.is_contiguous() and scale.is_contiguous()
     tiled = torch.empty(tiled_size(n, k, bits), dtype=torch.uint8, device=codes.device)
-    with torch.cuda.device(codes.device):
+    with _on(codes.device):
         check(lib().fdk_repack(codes.data_ptr(), scale.data_ptr(), n, k, bits, block_size, tiled.data_ptr(), _stream()))
     return tiled
 
@@ -251,7 +261,7 @@ def unpack(tiled: Tensor, n: int, k: int, bits: int, block_size: int, dtype: tor
     _require_cuda(tiled)
     codes = torch.empty((n, k * bits // 8), dtype=torch.uint8, device=tiled.device)
     scale = torch.empty((n, k // block_size), dtype=dtype, device=tiled.device)
-    with torch.cuda.device(tiled.device):
+    with _on(tiled.device):
         check(lib().fdk_unpack(tiled.data_ptr(), n, k, bits, block_size, codes.data_ptr(), scale.data_ptr(), _stream()))
     return codes, scale
 
@@ -263,7 +273,7 @@ def dequantise(codes: Tensor, lut: Tensor, scale: Tensor, bits: int) -> Tensor:
     block_size = k // scale.shape[1]
     assert lut.dtype == scale.dtype and all(t.is_contiguous() for t in (codes, lut, scale))
     w = torch.empty((n, k), dtype=scale.dtype, device=codes.device)
-    with torch.cuda.device(codes.device):
+    with _on(codes.device):
         check(
             lib().fdk_dequantise(
                 codes.data_ptr(), lut.data_ptr(), scale.data_ptr(), n, k, bits, block_size,
@@ -276,7 +286,7 @@ def dequantise(codes: Tensor, lut: Tensor, scale: Tensor, bits: int) -> Tensor:
 def dequantise_tiled(tiled: Tensor, lut: Tensor, n: int, k: int, bits: int) -> Tensor:
     _require_cuda(tiled, lut)
     w = torch.empty((n, k), dtype=lut.dtype, device=tiled.device)
-    with torch.cuda.device(tiled.device):
+    with _on(tiled.device):
         check(lib().fdk_dequantise_tiled(tiled.data_ptr(), lut.data_ptr(), n, k, bits, dtype_code(lut.dtype), w.data_ptr(), _stream()))
     return w
 
@@ -345,18 +355,17 @@ def linear_lut(
     """out[m, n] = x[m, k] @ W.T, W never materialised.  Writes `out` in place.  silu_pairs: W's
     rows alternate 32 gate rows and their 32 up rows, out[m, n / 2] = silu(gate) * up (m <= 16)."""
     _require_cuda(x, tiled, lut, out)
-    m = x.shape[0]
-    ws = workspace(x.device)
     if lut_bytes is None:
         lut_bytes = host_lut(lut)
-    with torch.cuda.device(x.device):
-        check(
-            lib().fdk_linear_lut(
-                x.data_ptr(), tiled.data_ptr(), lut.data_ptr(), lut_bytes, out.data_ptr(), m, n, k, bits,
-                dtype_code(x.dtype), ws.data_ptr(), ws.numel(),
-                (FLAG_PDL if pdl else 0) | (FLAG_SILU_PAIRS if silu_pairs else 0), _stream(),
-            )
+    ws = workspace(x.device)
+    with _on(x.device):
+        status = lib().fdk_linear_lut(
+            x.data_ptr(), tiled.data_ptr(), lut.data_ptr(), lut_bytes, out.data_ptr(), x.shape[0], n, k, bits,
+            dtype_code(x.dtype), ws.data_ptr(), ws.numel(),
+            (FLAG_PDL if pdl else 0) | (FLAG_SILU_PAIRS if silu_pairs else 0), _stream(),
         )
+    if status != OK:
+        check(status)
 
 
 def linear_lut_host(
@@ -372,7 +381,7 @@ def linear_lut_host(
     ws = workspace(tiled.device)
     if lut_bytes is None:
         lut_bytes = host_lut(lut)
-    with torch.cuda.device(tiled.device):
+    with _on(tiled.device):
         check(
             lib().fdk_linear_lut_host(
                 x_host.data_ptr(), tiled.data_ptr(), lut.data_ptr(), lut_bytes, out_host.data_ptr(), m, n, k, bits,
@@ -418,7 +427,7 @@ def linear_lut_fused(
     ws = workspace(tiled.device)
     if lut_bytes is None:
         lut_bytes = host_lut(lut)
-    with torch.cuda.device(tiled.device):
+    with _on(tiled.device):
         check(
             lib().fdk_linear_lut_fused(
                 None if x is None else x.data_ptr(), tiled.data_ptr(), lut.data_ptr(), lut_bytes,
@@ -432,7 +441,7 @@ def rope_table(pos: Tensor, table: Tensor, theta: float) -> None:
     """table[64] int32 = {bf16 cos, bf16 sin} of the rotary angles at position `pos` (device int64)."""
     _require_cuda(pos, table)
     assert pos.dtype == torch.int64 and table.dtype == torch.int32 and table.numel() == 64
-    with torch.cuda.device(pos.device):
+    with _on(pos.device):
         check(lib().fdk_rope_table(pos.data_ptr(), table.data_ptr(), theta, _stream()))
 
 
@@ -444,7 +453,7 @@ def norm_prepare(h: Tensor, weight: Tensor, x: Tensor, sumsq: Tensor) -> None:
     assert h.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and x.dtype == torch.bfloat16
     assert h.is_contiguous() and x.is_contiguous() and x.shape == h.shape and weight.numel() == width
     assert sumsq.dtype == torch.float32 and sumsq.shape == (rows, (width + 63) // 64)
-    with torch.cuda.device(h.device):
+    with _on(h.device):
         check(lib().fdk_norm_prepare(h.data_ptr(), weight.data_ptr(), x.data_ptr(), sumsq.data_ptr(), rows, width, _stream()))
 
 
@@ -453,7 +462,7 @@ def sumsq_tiles(h: Tensor, sumsq: Tensor) -> None:
     _require_cuda(h, sumsq)
     rows, width = h.shape
     assert sumsq.dtype == torch.float32 and sumsq.shape == (rows, (width + 63) // 64)
-    with torch.cuda.device(h.device):
+    with _on(h.device):
         check(lib().fdk_sumsq_tiles(h.data_ptr(), sumsq.data_ptr(), rows, width, _stream()))
 
 
@@ -461,7 +470,7 @@ def rmsnorm(h: Tensor, delta: Tensor | None, weight: Tensor, out: Tensor, eps: f
     """h += delta (when given, in place), out = RMSNorm(h) * weight.  bf16 [rows, width]."""
     _require_cuda(h, weight, out)
     rows, width = h.shape
-    with torch.cuda.device(h.device):
+    with _on(h.device):
         check(
             lib().fdk_rmsnorm(
                 h.data_ptr(), None if delta is None else delta.data_ptr(), weight.data_ptr(), out.data_ptr(),
@@ -484,14 +493,14 @@ def tp_buffer_create(nbytes: int, device: torch.device) -> tuple[int, bytes]:
     """Zeroed device buffer that other processes can map -> (device pointer, 64-byte handle)."""
     ptr = ctypes.c_void_p()
     handle = ctypes.create_string_buffer(64)
-    with torch.cuda.device(device):
+    with _on(device):
         check(lib().fdk_tp_buffer_create(nbytes, ctypes.byref(ptr), handle))
     return ptr.value, handle.raw
 
 
 def tp_buffer_open(handle: bytes, device: torch.device) -> int:
     ptr = ctypes.c_void_p()
-    with torch.cuda.device(device):
+    with _on(device):
         check(lib().fdk_tp_buffer_open(handle, ctypes.byref(ptr)))
     return ptr.value
 
@@ -528,7 +537,7 @@ def linear_lut_push(
     ws = workspace(x.device)
     if lut_bytes is None:
         lut_bytes = host_lut(lut)
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         check(
             lib().fdk_linear_lut_push(
                 x.data_ptr(), tiled.data_ptr(), lut.data_ptr(), lut_bytes, m, n, k, bits,
@@ -541,7 +550,7 @@ def rmsnorm_reduce(h: Tensor, ex: TpExchange, weight: Tensor, out: Tensor, eps: 
     """h += sum over ranks of the latest push (in place), out = RMSNorm(h) * weight."""
     _require_cuda(h, weight, out)
     rows, width = h.shape
-    with torch.cuda.device(h.device):
+    with _on(h.device):
         check(
             lib().fdk_rmsnorm_reduce(
                 h.data_ptr(), ctypes.byref(ex), weight.data_ptr(), out.data_ptr(), rows, width, eps, _stream(),
@@ -558,7 +567,7 @@ def rope_append(
     in the row order of the projection kernel's rotary output ([0..31, 64..95, 32..63, 96..127])."""
     _require_cuda(qkv, pos, q_out, k_cache, v_cache)
     assert pos.dtype == torch.int64
-    with torch.cuda.device(qkv.device):
+    with _on(qkv.device):
         check(
             (lib().fdk_rope_append_paired if paired else lib().fdk_rope_append)(
                 qkv.data_ptr(), pos.data_ptr(), q_out.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),
@@ -577,7 +586,7 @@ def rope_prefill(qkv: Tensor, table: Tensor, q_out: Tensor, k_cache: Tensor, v_c
     assert all(t.is_contiguous() and t.dtype == torch.bfloat16 for t in (qkv, table, q_out, k_cache, v_cache))
     assert qkv.shape == (batch * tokens, (q_heads + 2 * kv_heads) * 128) and table.shape == (tokens, 64, 2)
     assert k_cache.shape == v_cache.shape == (batch, kv_heads, max_len, 128)
-    with torch.cuda.device(qkv.device):
+    with _on(qkv.device):
         check(
             lib().fdk_rope_prefill_paired(
                 qkv.data_ptr(), table.data_ptr(), q_out.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),
@@ -591,7 +600,7 @@ def silu_mul(gate_up: Tensor, out: Tensor, group: int | None = None) -> None:
     (default: all gates, then all ups)."""
     _require_cuda(gate_up, out)
     rows, width = out.shape
-    with torch.cuda.device(out.device):
+    with _on(out.device):
         check(lib().fdk_silu_mul(gate_up.data_ptr(), out.data_ptr(), rows, width, width if group is None else group, _stream()))
 
 
@@ -619,14 +628,14 @@ def argmax(x: Tensor, out: Tensor) -> None:
     """out[r] = argmax of row r of x [rows, n] (bf16 or fp16; lowest index among equals)."""
     _require_cuda(x, out)
     assert x.dim() == 2 and x.is_contiguous() and out.dtype == torch.int64 and out.is_contiguous() and out.numel() == x.shape[0]
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         check(lib().fdk_argmax(x.data_ptr(), out.data_ptr(), x.shape[0], x.shape[1], dtype_code(x.dtype), _stream()))
 
 
 def attention_status(counters: Tensor, batch: int, kv_heads: int) -> int:
     """Status word of a decode-attention scratch (synchronises): 0, or 1 after a wait ran out."""
     out = ctypes.c_int(0)
-    with torch.cuda.device(counters.device):
+    with _on(counters.device):
         check(lib().fdk_decode_attention_status(counters.data_ptr(), batch, kv_heads, ctypes.byref(out)))
     return out.value
 
@@ -635,7 +644,7 @@ def decode_attention(q: Tensor, k_cache: Tensor, v_cache: Tensor, pos: Tensor, o
                      scratch: Tensor, counters: Tensor, q_heads: int, kv_heads: int, splits: int) -> None:
     """One query token per batch row against the KV cache [batch, kv_heads, max_len, 128], keys 0..pos."""
     _require_cuda(q, k_cache, v_cache, pos, out)
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         check(
             lib().fdk_decode_attention(
                 q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), pos.data_ptr(), out.data_ptr(),
