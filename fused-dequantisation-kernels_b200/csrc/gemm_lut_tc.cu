@@ -4,7 +4,7 @@
 // block by block in tensor memory and never written to HBM.
 //
 // Persistent, one CTA per SM.  The product is cut into tiles of 128 weight rows (MMA M) by up to
-// 256 batch rows (MMA N); the slabs of all tiles form one sequence, of which each CTA owns a
+// 192 batch rows (MMA N); the slabs of all tiles form one sequence, of which each CTA owns a
 // contiguous range, so every SM has the same work whatever the sizes.  A tile that is cut by a
 // range boundary belongs to the CTA with its first slabs; the others park their fp32 sums in the
 // workspace.  24 warps, specialised:
@@ -24,7 +24,7 @@
 // the store of the tile and the MMA's reads of it out of shared memory, and its MMAs of
 // small N are faster (a block at N = 32 takes 68 cycles, 161 with A in shared memory).  Before (A in
 // shared memory, eight dequantising warps, a tile per CTA) and now, 4 bits: 48 rows of 11264 x 3072 23.1 ->
-// 12.0 us; 2048 rows of 28672 x 4096 791 -> 370 us (1.30 PFLOP/s).  Tried and not kept: groups
+// 12.0 us; 2048 rows of 28672 x 4096 791 -> 352 us (1.37 PFLOP/s).  Tried and not kept: groups
 // of four blocks per copy, barrier and stage (18.4 us at 32 rows of 8192^2 against 16.7: a set
 // then waits for a whole group, and the larger stages leave fewer of them).
 // Every wait is bounded; one that runs out sets a status bit, and the kernel still frees its
@@ -47,13 +47,17 @@ constexpr int kTcWarps = kTcDequantWarps + kTcEpilogueWarps + kTcCodeWarps + 2;
 constexpr int kTcXWarp = kTcWarps - 2, kTcMmaWarp = kTcWarps - 1, kTcFirstCodeWarp = kTcXWarp - kTcCodeWarps;
 constexpr int kTcThreads = 32 * kTcWarps;
 constexpr int kTcTileRows = 128;
-constexpr int kTcMaxBatch = 256;     // MMA N limit
+// Batch rows of a tile (MMA N, at most 256).  With 192 two accumulators and four A stages fit tensor memory,
+// so a tile's epilogue overlaps the next tile; with 256 it does not: 4 bits, 1000 rows of 5120 x 3072
+// 35.9 us against 30.8, 256 of 3072^2 20.9 / 13.6, 2048 of 28672 x 4096 366 / 352.  128: 31.4, 13.6, 388.
+constexpr int kTcMaxBatch = 192;
 constexpr int kTcMaxStages = 8;
 constexpr int kTcMaxCodeSlots = 16;
 constexpr int kTcTmemColumns = 512;
+constexpr int kTcAccumulators = 2;
 constexpr int kTcFlagsPerRank = (kTcMaxBatch / 16) * 4;  // 16 batch columns x 32 weight rows each
 // rows of the lookup table 256 bytes apart: a lookup address is one PRMT.  8 bits: no room beside
-// 256 batch rows and four slabs
+// 128 batch rows and four slabs
 template <int BITS>
 constexpr bool kTcWideTable = BITS == 1 || BITS == 2 || BITS == 4;
 constexpr int kTcStatusTimeout = 1;
@@ -69,7 +73,6 @@ struct TcParams {
   int row_tiles;          // 64-row tiles of the tiled buffer
   int k_blocks, k_slabs;  // k / 64; slabs per 64-row tile
   int stages_log2, code_slots;
-  int acc_slots;          // accumulators in tensor memory: 2 where both fit beside the A stages
   int split;              // ranges may cut tiles
   float* partial;         // [rank][n_tile][128] fp32 sums of a CTA that does not own its first tile
   int* flags;             // [rank][column sixteenth][row quarter] 1: published; the reader clears it again
@@ -313,7 +316,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       mbar_init(c_full + 8 * c, 1);
       mbar_init(c_empty + 8 * c, KSB == 1 ? 4 : kTcDequantWarps);  // one set, or all
     }
-    for (int a = 0; a < 2; ++a) {
+    for (int a = 0; a < kTcAccumulators; ++a) {
       mbar_init(acc_full + 8 * a, 1);
       mbar_init(acc_empty + 8 * a, kTcEpilogueWarps);
     }
@@ -432,7 +435,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   auto last_epilogue = [&](int part) {
     if (!mbar_wait(acc_last, 0)) timed_out = true;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    epilogue(last_tile, last_begin, last_end, acc_base + (segments - 1) % p.acc_slots * p.n_tile, part, kSets + 1);
+    epilogue(last_tile, last_begin, last_end, acc_base + (segments - 1) % kTcAccumulators * p.n_tile, part, kSets + 1);
   };
 
   if (segments == 0) {
@@ -482,9 +485,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     const uint32_t idesc = (1u << 4) | (kFormat << 7) | (kFormat << 10) | ((uint32_t)(p.n_tile >> 3) << 17) | ((128u >> 4) << 24);
     int i = 0, ks = u0 % p.k_slabs;
     for (int seg = 0, u = u0; seg < segments && !timed_out; ++seg) {
-      const int a = seg % p.acc_slots;
+      const int a = seg % kTcAccumulators;
       const uint32_t acc = acc_base + a * p.n_tile;
-      if (!mbar_wait(acc_empty + 8 * a, ((seg / p.acc_slots) & 1) ^ 1)) { timed_out = true; break; }
+      if (!mbar_wait(acc_empty + 8 * a, ((seg / kTcAccumulators) & 1) ^ 1)) { timed_out = true; break; }
       uint32_t accumulate = 0;
       for (bool more = true; more && !timed_out;) {
         const int nb = blocks_of(ks);
@@ -518,8 +521,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     int u = u0;
     for (int seg = 0; seg + 1 < segments; ++seg) {
       const int tile = u / p.k_slabs, begin = u - tile * p.k_slabs;
-      const int a = seg % p.acc_slots;
-      if (!mbar_wait(acc_full + 8 * a, (seg / p.acc_slots) & 1)) timed_out = true;
+      const int a = seg % kTcAccumulators;
+      if (!mbar_wait(acc_full + 8 * a, (seg / kTcAccumulators) & 1)) timed_out = true;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       epilogue(tile, begin, p.k_slabs, acc_base + a * p.n_tile, 0, 1);
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -726,9 +729,8 @@ int gemm_lut_tc(const void* x, const void* tiled, const void* lut, const void* l
   const long long tiles = (long long)((n + kTcTileRows - 1) / kTcTileRows) * p.m_tiles, units = tiles * d.k_slabs;
   FDK_CHECK_ARG(units < (1ll << 31), FDK_ERR_SHAPE, "m=%d, n=%d, k=%d: too many tiles", m, n, k);
   p.tiles = (int)tiles;
-  // up to 128 batch rows eight A stages and two accumulators fit tensor memory, up to 192 four and two
+  // eight A stages fit tensor memory beside two accumulators of 128 columns, four beside two of 192
   p.stages_log2 = p.n_tile <= 128 ? 3 : 2;
-  p.acc_slots = p.n_tile <= 192 ? 2 : 1;
   p.flags = (int*)((uint8_t*)workspace + kTcFlagsOffset);
   p.partial = (float*)((uint8_t*)workspace + kTcPartialOffset);
   // One CTA per SM.  Ranges cut tiles where the workspace has room for every CTA's partial sums.

@@ -237,7 +237,7 @@ __device__ __forceinline__ int ld_relaxed_s32(const int* p) {
 //   [0, 16 KB)            use counts of split row tiles (4095 ints) + the status word
 //   [16 KB, kGemvEnd)     tagged partial sums of the GEMV kernel, 8 KB per SM, room for 160 SMs
 //   then 40 KB of flags of the tensor-core GEMM (64 per CTA; zero between launches)
-//   then its fp32 partial tiles: one of 128 rows x up to 256 batch columns per CTA, room for 148
+//   then its fp32 partial tiles, one per CTA: room for 148 of 128 rows x 256 batch columns
 constexpr size_t kCounterBytes = 16384;
 constexpr int kStatusWord = 4095;
 constexpr size_t kGemvEnd = kCounterBytes + (size_t)160 * 1024 * sizeof(uint2);
