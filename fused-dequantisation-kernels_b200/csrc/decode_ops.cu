@@ -245,10 +245,11 @@ __global__ void rope_append_kernel(const uint16_t* __restrict__ qkv, const long 
 
 // Rotary embedding of a whole prompt, and its keys and values into the caches: qkv [batch * T, heads * 128]
 // (q and k heads in the paired order, see above), table [T][64] of {bf16 cos, bf16 sin} -> q
-// [batch, q_heads, T, 128] and positions 0 .. T - 1 of the caches.  The values of rope_append_kernel.
+// [batch, T, q_heads, 128] and positions 0 .. T - 1 of the caches.  The values of rope_append_kernel.
 // Bound by HBM (every value read and written once); a thread takes eight of the 64 pairs of a
 // head, two 16-byte vectors each way, neighbouring threads neighbouring vectors.  1000 tokens of 24 + 2 x
-// 8 heads: replaces about 25 framework launches a layer.
+// 8 heads: 7.9 us, in the place of about 25 framework launches a layer.  q is written in the order of the
+// projection's rows: the attention then returns its result in that order too (10.7 us of copying less).
 __global__ void rope_prefill_kernel(const uint16_t* __restrict__ qkv, const uint32_t* __restrict__ table,
                                     uint16_t* __restrict__ q_out, uint16_t* __restrict__ k_cache,
                                     uint16_t* __restrict__ v_cache, int t_count, int q_heads, int kv_heads, int max_len,
@@ -290,7 +291,7 @@ __global__ void rope_prefill_kernel(const uint16_t* __restrict__ qkv, const uint
       lo[j] = out0[0] | (out0[1] << 16);
       hi[j] = out1[0] | (out1[1] << 16);
     }
-    uint16_t* dst = head < q_heads ? q_out + ((b * q_heads + head) * t_count + t) * 128
+    uint16_t* dst = head < q_heads ? q_out + (row * q_heads + head) * 128
                                    : k_cache + ((b * kv_heads + (head - q_heads)) * max_len + t) * 128;
     *reinterpret_cast<uint4*>(dst + i) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
     *reinterpret_cast<uint4*>(dst + i + 64) = make_uint4(hi[0], hi[1], hi[2], hi[3]);

@@ -368,14 +368,14 @@ class LlamaDecoder(nn.Module):
         inv_freq = 1.0 / (dims.rope_theta ** (torch.arange(0, 128, 2, dtype=torch.float32, device=dev) / 128))
         angles = torch.arange(t, dtype=torch.float32, device=dev)[:, None] * inv_freq[None, :]
         table = torch.stack((angles.cos(), angles.sin()), dim=-1).bfloat16()  # [T, 64, 2]
-        q = torch.empty((batch, self.q_heads, t, 128), device=dev, dtype=torch.bfloat16)
+        q = torch.empty((batch, t, self.q_heads, 128), device=dev, dtype=torch.bfloat16)
 
         delta = None
         for i, layer in enumerate(self.layers):
             native.rmsnorm(hidden, delta, layer.input_norm, normed, eps)
             native.rope_prefill(layer.qkv(normed), table, q, self.k_cache[i], self.v_cache[i])
             attn = nn.functional.scaled_dot_product_attention(
-                q, self.k_cache[i][:, :, :t], self.v_cache[i][:, :, :t], is_causal=True, enable_gqa=True
+                q.transpose(1, 2), self.k_cache[i][:, :, :t], self.v_cache[i][:, :, :t], is_causal=True, enable_gqa=True
             ).transpose(1, 2).reshape(rows, self.q_heads * 128).contiguous()
             delta = layer.o(attn)
             self.tp.all_reduce(delta)

@@ -578,10 +578,10 @@ def rope_append(
 
 def rope_prefill(qkv: Tensor, table: Tensor, q_out: Tensor, k_cache: Tensor, v_cache: Tensor) -> None:
     """Rotary embedding of a prompt's fused q|k|v projections [batch * T, heads * 128] (q and k heads in the
-    paired row order): q_out [batch, q_heads, T, 128], k and v to positions 0 .. T - 1 of the caches
+    paired row order): q_out [batch, T, q_heads, 128], k and v to positions 0 .. T - 1 of the caches
     [batch, kv_heads, max_len, 128].  table [T, 64, 2]: cosines and sines."""
     _require_cuda(qkv, table, q_out, k_cache, v_cache)
-    batch, q_heads, tokens, _ = q_out.shape
+    batch, tokens, q_heads, _ = q_out.shape
     kv_heads, max_len = k_cache.shape[1:3]
     assert all(t.is_contiguous() and t.dtype == torch.bfloat16 for t in (qkv, table, q_out, k_cache, v_cache))
     assert qkv.shape == (batch * tokens, (q_heads + 2 * kv_heads) * 128) and table.shape == (tokens, 64, 2)
