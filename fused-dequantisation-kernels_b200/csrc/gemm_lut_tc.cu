@@ -392,7 +392,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             }
             *f = 0;
           }
-          timed_out = __any_sync(0xffffffffu, timed_out);  // also orders the other lanes' reads after the flags
+          timed_out = __any_sync(0xffffffffu, timed_out);
+          __syncwarp();  // the lanes' reads below come after every polling lane's acquire (a vote orders no memory)
           // in rank order; two shares' loads are in flight at a time
           for (int o = rank + 1; o <= last_rank; o += 2) {
             const float* theirs = p.partial + o * slot + at;
