@@ -28,7 +28,9 @@
 // of four blocks per copy, barrier and stage (18.4 us at 32 rows of 8192^2 against 16.7: a set
 // then waits for a whole group, and the larger stages leave fewer of them).
 // Every wait is bounded; one that runs out sets a status bit, and the kernel still frees its
-// tensor memory and returns.
+// tensor memory and returns.  Under programmatic launch the bounds count this kernel's own time only: a
+// role waits for the kernel before (griddepcontrol.wait, which has no bound) ahead of its first bounded
+// wait that x, and so that kernel, can hold up.
 #include <cuda.h>
 
 #include <cmath>
@@ -459,7 +461,11 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         if (second) bulk_copy(dst + (uint32_t)L::kSlabBytes, src + tile_bytes, L::kSlabBytes, bar);
       }
       for (int i = 0; i < kTcCodeWarps; ++i) c.next(p);
-      if ((slot += kTcCodeWarps) >= p.code_slots) { slot -= p.code_slots; phase ^= 1; }
+      if ((slot += kTcCodeWarps) >= p.code_slots) {
+        slot -= p.code_slots;
+        phase ^= 1;
+        asm volatile("griddepcontrol.wait;" ::: "memory");  // from here on a slot is freed by way of x
+      }
     }
   } else if (warp == kTcXWarp) {
     // ---------------- x producer ----------------
@@ -480,6 +486,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     }
   } else if (warp == kTcMmaWarp) {
     // ---------------- MMA issuer ----------------
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // a stage is full once x is in it
     // instruction descriptor: fp32 accumulate, A and B both bf16 (format 1) or both fp16
     // (format 0), both K-major, N = n_tile, M = 128
     constexpr uint32_t kFormat = FP16 ? 0u : 1u;
@@ -549,6 +556,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     // of four); the other slabs are seen by every warp.
     int u = KSB == 1 ? u0 + set : u0, slot = KSB == 1 ? set : 0, c_phase = 0;
     int ks = KSB == 1 ? 0 : u0 % p.k_slabs, i = 0;
+    // Second uses of a code slot or stage wait for MMAs, hence for x; the first ones do not, and fill
+    // tensor memory while the kernel before is still running.
+    auto wait_for_x = [&] { asm volatile("griddepcontrol.wait;" ::: "memory"); };
     auto fetch = [&](RowCodes<BITS>& codes, uint32_t& s2) -> int {
       while (u < u1) {
         const int nb = KSB == 1 ? 1 : blocks_of(ks);
@@ -567,12 +577,12 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         if constexpr (KSB == 1) {
           u += kSets;
           slot += kSets;
-          if (slot >= p.code_slots) { slot -= p.code_slots; c_phase ^= 1; }
+          if (slot >= p.code_slots) { slot -= p.code_slots; c_phase ^= 1; wait_for_x(); }
         } else {
           ++u;
           i += nb;
           if (++ks == p.k_slabs) ks = 0;
-          if (++slot == p.code_slots) { slot = 0; c_phase ^= 1; }
+          if (++slot == p.code_slots) { slot = 0; c_phase ^= 1; wait_for_x(); }
         }
         if (mine) return block;
       }
@@ -595,6 +605,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       codes.template decode<0, FP16, WIDE>(lane_base, s2, v, 0);
       codes.template decode<1, FP16, WIDE>(lane_base, s2, v, 8);
       if (stored >= 0) hand_over(stored);
+      if (block == S + set) wait_for_x();  // the set's first second use
       if (!mbar_wait(empty + 8 * s, ((block >> p.stages_log2) & 1) ^ 1)) { timed_out = true; break; }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       tmem_store16(a_lane + 32 * s, v);

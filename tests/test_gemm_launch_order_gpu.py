@@ -1,0 +1,68 @@
+"""The tensor-core GEMM between the kernels of its stream, under programmatic dependent launch."""
+
+import ctypes
+import shutil
+import subprocess
+
+import pytest
+import torch
+
+from fdk import models, native
+
+pytestmark = pytest.mark.gpu
+
+# Lets the next kernel start, stays busy for a while (bounded by its clock and by a count), then writes x.
+SLOW_PRODUCER = r"""
+#include <cuda_runtime.h>
+__global__ void slow_producer(const uint4* src, uint4* dst, int vectors, unsigned long long ns) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  unsigned long long t0, now;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+  for (unsigned i = 0; i < 100000000u; ++i) {
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+    if (now - t0 > ns) break;
+    __nanosleep(1000);
+  }
+  for (int i = threadIdx.x; i < vectors; i += blockDim.x) dst[i] = src[i];
+}
+extern "C" int launch_slow_producer(const void* src, void* dst, int vectors, unsigned long long ns, void* stream) {
+  slow_producer<<<1, 256, 0, (cudaStream_t)stream>>>((const uint4*)src, (uint4*)dst, vectors, ns);
+  return (int)cudaGetLastError();
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def slow_producer(tmp_path_factory):
+    folder = tmp_path_factory.mktemp("slow_producer")
+    source, library = folder / "slow_producer.cu", folder / "slow_producer.so"
+    source.write_text(SLOW_PRODUCER)
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-Xcompiler", "-fPIC",
+                    "-o", str(library), str(source)], check=True)
+    fn = ctypes.CDLL(str(library)).launch_slow_producer
+    fn.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_ulonglong, ctypes.c_void_p]
+    return fn
+
+
+@pytest.mark.parametrize("m,bits", [(32, 4), (200, 8), (32, 1), (100, 3)])
+def test_bounded_waits_do_not_count_the_kernel_before(slow_producer, m, bits):
+    """The kernel before takes longer than the two seconds after which a wait gives up, and hands over x only
+    then: no wait runs out, and the result is that of a launch in plain order.  Every CTA's share is longer than its
+    rings of code slots and stages, so that every role reaches its second uses."""
+    n, k = 11264, 16384
+    gen = torch.Generator(device="cuda").manual_seed(m + bits)
+    w = (torch.randn((n, k), generator=gen, device="cuda") * k**-0.5).bfloat16()
+    layer = models.QuantisedLinear.create(w, models.QuantisationConfig(bits, 64))
+    source = torch.randn((m, k), generator=gen, device="cuda").bfloat16()
+    args = (layer.tiled(), layer.lut)
+    want = torch.empty((m, n), device="cuda", dtype=torch.bfloat16)
+    native.linear_lut(source, *args, want, n, k, bits)
+    x, got = torch.full_like(source, float("nan")), torch.empty_like(want)
+    torch.cuda.synchronize()
+    assert slow_producer(source.data_ptr(), x.data_ptr(), x.numel() // 8, 2_600_000_000, native._stream()) == 0
+    native.linear_lut(x, *args, got, n, k, bits, pdl=True)
+    torch.cuda.synchronize()
+    assert native.device_status() == 0
+    assert torch.equal(got, want)
