@@ -112,6 +112,13 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// Stands between a repack and the launches after it.  A projection launched with FDK_FLAG_PDL reads the
+// tiled buffer before it waits for the kernel before it; were that the repack, its stores need not be
+// visible yet (it is over, or the projection would not have started, but only a wait or the plain
+// order of a stream makes its stores visible).  This kernel follows the repack in plain order, and whatever
+// comes next starts after it.
+__global__ void repacked_kernel() {}
+
 template <int BITS>
 int launch_repack(const void* codes, const void* scale, void* tiled, int n, int k, int block_size, cudaStream_t stream) {
   const TiledDims d = tiled_dims(n, k, BITS);
@@ -120,6 +127,8 @@ int launch_repack(const void* codes, const void* scale, void* tiled, int n, int 
   repack_kernel<BITS><<<pairs < 148 * 32 ? pairs : 148 * 32, 256, 0, stream>>>(
       (const uint8_t*)codes, (const uint16_t*)scale, (uint8_t*)tiled, n, k, block_size / kBlock, d,
       (uintptr_t)codes % kAlign == 0);
+  FDK_CUDA(cudaGetLastError());
+  repacked_kernel<<<1, 32, 0, stream>>>();
   FDK_CUDA(cudaGetLastError());
   return FDK_OK;
 }

@@ -66,3 +66,43 @@ def test_bounded_waits_do_not_count_the_kernel_before(slow_producer, m, bits):
     torch.cuda.synchronize()
     assert native.device_status() == 0
     assert torch.equal(got, want)
+
+
+class EdgeData(ctypes.Structure):
+    """`cudaGraphEdgeData`; type 1 is a programmatic dependency, 0 a full one."""
+
+    _fields_ = [("from_port", ctypes.c_ubyte), ("to_port", ctypes.c_ubyte), ("type", ctypes.c_ubyte), ("reserved", ctypes.c_ubyte * 5)]
+
+
+def graph_edges(graph: int) -> list[tuple[int, int, bool]]:
+    """(node, its successor, whether the successor may start before the node has completed) of a captured graph."""
+    get = ctypes.CDLL("libcudart.so.12").cudaGraphGetEdges_v2
+    count = ctypes.c_size_t(0)
+    assert get(ctypes.c_void_p(graph), None, None, None, ctypes.byref(count)) == 0
+    sources, targets = ((ctypes.c_void_p * count.value)() for _ in range(2))
+    data = (EdgeData * count.value)()
+    assert get(ctypes.c_void_p(graph), sources, targets, data, ctypes.byref(count)) == 0
+    return [(a, b, e.type == 1) for a, b, e in zip(sources, targets, data)]
+
+
+@pytest.mark.parametrize("m", [1, 8, 32])
+def test_no_launch_reads_a_tiled_buffer_early_that_the_kernel_before_wrote(m):
+    """The first call of a layer repacks its weight and launches the projection, which reads codes before it waits
+    for its predecessor.  Captured and not run: the repack's successor depends on it in full, and the
+    projection's early start is on a kernel that wrote nothing."""
+    layer = models.QuantisedLinear.create(torch.randn((256, 512), device="cuda").bfloat16(), models.QuantisationConfig(4, 64))
+    x = torch.randn((m, 512), device="cuda").bfloat16()
+    graph, stream = torch.cuda.CUDAGraph(keep_graph=True), torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        layer.tiled()
+        stream.synchronize()
+        layer(x)  # the stream's workspace and the host copy of the table
+        stream.synchronize()
+        layer._tiled_key = None  # as after a change of the weight
+        with torch.cuda.graph(graph, stream=stream):
+            layer(x)
+    edges = graph_edges(graph.raw_cuda_graph())
+    (repack,) = {a for a, _, _ in edges} - {b for _, b, _ in edges}  # the first kernel
+    assert not any(programmatic for a, _, programmatic in edges if a == repack), edges
+    assert any(programmatic for _, _, programmatic in edges), edges
