@@ -7,7 +7,8 @@
 // 192 batch rows (MMA N); the slabs of all tiles form one sequence, of which each CTA owns a
 // contiguous range, so every SM has the same work whatever the sizes.  A tile that is cut by a
 // range boundary belongs to the CTA with its first slabs; the others park their fp32 sums in the
-// workspace.  24 warps, specialised:
+// workspace, under flags that hold the number of the launch: a flag that an earlier launch left, whatever
+// became of that launch, is never taken for one of this.  24 warps, specialised:
 //   warps 0..15  dequantise, in four sets of four warps; set s takes the 64-column blocks
 //                s, s + 4, ...: code bytes from shared memory -> replicated table lookup ->
 //                times the block scale -> tcgen05.st into the stage's A tile in TENSOR memory;
@@ -57,7 +58,10 @@ constexpr int kTcMaxStages = 8;
 constexpr int kTcMaxCodeSlots = 16;
 constexpr int kTcTmemColumns = 512;
 constexpr int kTcAccumulators = 2;
-constexpr int kTcFlagsPerRank = (kTcMaxBatch / 16) * 4;  // 16 batch columns x 32 weight rows each
+static_assert(kTcFlagsPerRank == (kTcMaxBatch / 16) * 4, "a flag per 16 batch columns x 32 weight rows");
+// Launches counted in the workspace: every CTA adds one at its end, rank 0 also what is missing to 2^16, so that
+// the count above the low 16 bits moves on when the last CTA has added.
+constexpr int kTcLaunchShift = 16;
 // rows of the lookup table 256 bytes apart: a lookup address is one PRMT.  8 bits: no room beside
 // 128 batch rows and four slabs
 template <int BITS>
@@ -77,7 +81,8 @@ struct TcParams {
   int stages_log2, code_slots;
   int split;              // ranges may cut tiles
   float* partial;         // [rank][n_tile][128] fp32 sums of a CTA that does not own its first tile
-  int* flags;             // [rank][column sixteenth][row quarter] 1: published; the reader clears it again
+  int* flags;             // [rank][column sixteenth][row quarter] the launch that published
+  unsigned long long* launches;  // launches on this workspace with cut tiles
   uint32_t smem_base, table_addr, bar_addr;
   uint32_t b_addr[kTcMaxStages], c_addr[kTcMaxCodeSlots];
 };
@@ -302,7 +307,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   const int S = 1 << p.stages_log2;
   const uint32_t full = p.bar_addr, empty = full + 8 * kTcMaxStages,
                  c_full = empty + 8 * kTcMaxStages, c_empty = c_full + 8 * kTcMaxCodeSlots,
-                 acc_full = c_empty + 8 * kTcMaxCodeSlots, acc_empty = acc_full + 16, acc_last = acc_empty + 16, tmem_slot = acc_last + 8;
+                 acc_full = c_empty + 8 * kTcMaxCodeSlots, acc_empty = acc_full + 16, acc_last = acc_empty + 16, tmem_slot = acc_last + 8,
+                 launch_slot = tmem_slot + 4;
   // Waits go to CTAs of lower block index, which the GPU starts first: rank r's successors in
   // the unit sequence are the blocks before it.
   const int rank = (int)gridDim.x - 1 - (int)blockIdx.x;
@@ -322,7 +328,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       mbar_init(acc_full + 8 * a, 1);
       mbar_init(acc_empty + 8 * a, kTcEpilogueWarps);
     }
-    mbar_init(acc_last, 1);
+    mbar_init(acc_last, 2);  // the last MMAs, and the launch number in shared memory
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -353,7 +359,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   auto blocks_of = [&](int ks) { return KSB == 1 ? 1 : min(KSB, p.k_blocks - ks * KSB); };
 
   // ---- epilogue of one tile segment [begin, end) of slabs, by `parts` warps per 32-row quarter ----
-  auto epilogue = [&](int tile, int begin, int end, uint32_t acc, int part, int parts) {
+  auto epilogue = [&](int tile, int begin, int end, uint32_t acc, int part, int parts, int launch) {
     const int nt = tile / p.m_tiles, mt = tile - nt * p.m_tiles;
     const int quarter = warp & 3;
     const int row = nt * kTcTileRows + 32 * quarter + 8 * (lane & 3) + (lane >> 2);
@@ -384,7 +390,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             for (uint32_t spin = 0;; ++spin) {
               int set;
               asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(set) : "l"(f) : "memory");
-              if (set != 0) break;
+              if (set == launch) break;
               if ((spin & 255u) == 255u) {
                 unsigned long long now;
                 asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
@@ -392,7 +398,6 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 else if (now - t0 > 2000000000ull) { timed_out = true; break; }
               }
             }
-            *f = 0;
           }
           timed_out = __any_sync(0xffffffffu, timed_out);
           __syncwarp();  // the lanes' reads below come after every polling lane's acquire (a vote orders no memory)
@@ -427,7 +432,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       __syncwarp();
       __threadfence();
       const int c0 = 16 * (part + lane * parts);
-      if (c0 < p.n_tile) asm volatile("st.relaxed.gpu.global.s32 [%0], %1;" ::"l"(flag(rank, c0)), "r"(1) : "memory");
+      if (c0 < p.n_tile) asm volatile("st.relaxed.gpu.global.s32 [%0], %1;" ::"l"(flag(rank, c0)), "r"(launch) : "memory");
     }
   };
   constexpr int kSets = kTcDequantWarps / 4;
@@ -438,7 +443,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   auto last_epilogue = [&](int part) {
     if (!mbar_wait(acc_last, 0)) timed_out = true;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    epilogue(last_tile, last_begin, last_end, acc_base + (segments - 1) % kTcAccumulators * p.n_tile, part, kSets + 1);
+    epilogue(last_tile, last_begin, last_end, acc_base + (segments - 1) % kTcAccumulators * p.n_tile, part, kSets + 1,
+             (int)ring32(launch_slot));
   };
 
   if (segments == 0) {
@@ -526,13 +532,23 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   } else if (warp >= kTcDequantWarps) {
     // ---------------- epilogue ----------------
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    int launch = 0;  // the same in every CTA: it moves on once all have read it
+    if (p.split) {
+      unsigned long long count;
+      asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(count) : "l"(p.launches) : "memory");
+      launch = (int)(count >> kTcLaunchShift) + 1;
+    }
+    if (warp == kTcDequantWarps && lane == 0) {  // for the warps that share the last epilogue
+      asm volatile("st.shared.u32 [%0], %1;" ::"r"(launch_slot), "r"(launch) : "memory");
+      mbar_arrive(acc_last);
+    }
     int u = u0;
     for (int seg = 0; seg + 1 < segments; ++seg) {
       const int tile = u / p.k_slabs, begin = u - tile * p.k_slabs;
       const int a = seg % kTcAccumulators;
       if (!mbar_wait(acc_full + 8 * a, (seg / kTcAccumulators) & 1)) timed_out = true;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      epilogue(tile, begin, p.k_slabs, acc_base + a * p.n_tile, 0, 1);
+      epilogue(tile, begin, p.k_slabs, acc_base + a * p.n_tile, 0, 1, launch);
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(acc_empty + 8 * a);
@@ -622,6 +638,12 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   if (timed_out && lane == 0) atomicOr(p.status, kTcStatusTimeout);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  // Every CTA of a launch that cuts tiles has units, so this thread has waited for the launch before, and
+  // every warp of the CTA has read the count.
+  if (p.split && threadIdx.x == 0)
+    asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(p.launches),
+                 "l"(rank == 0 ? (1ull << kTcLaunchShift) - (gridDim.x - 1) : 1ull)
+                 : "memory");
   if (warp == kTcMmaWarp) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)kTcTmemColumns) : "memory");
@@ -744,6 +766,7 @@ int gemm_lut_tc(const void* x, const void* tiled, const void* lut, const void* l
   // eight A stages fit tensor memory beside two accumulators of 128 columns, four beside two of 192
   p.stages_log2 = p.n_tile <= 128 ? 3 : 2;
   p.flags = (int*)((uint8_t*)workspace + kTcFlagsOffset);
+  p.launches = (unsigned long long*)((uint8_t*)workspace + kTcLaunchesOffset);
   p.partial = (float*)((uint8_t*)workspace + kTcPartialOffset);
   // One CTA per SM.  Ranges cut tiles where the workspace has room for every CTA's partial sums.
   // Where a tile is shared by many CTAs its owner reads all their sums (about 10 cycles per CTA and
@@ -761,7 +784,7 @@ int gemm_lut_tc(const void* x, const void* tiled, const void* lut, const void* l
     if (units < grid) grid = (int)units;
     if (grid < tiles) grid = (int)tiles;
   }
-  p.split = room >= (size_t)grid && grid * kTcFlagsPerRank * sizeof(int) <= kTcPartialOffset - kTcFlagsOffset;
+  p.split = room >= (size_t)grid;
   if (!p.split && tiles < grid) grid = (int)tiles;
   CUtensorMap map;
   const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)m};

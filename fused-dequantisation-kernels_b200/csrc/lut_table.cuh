@@ -236,13 +236,16 @@ __device__ __forceinline__ int ld_relaxed_s32(const int* p) {
 // ---- workspace layout (bytes) -----------------------------------------------------------------
 //   [0, 16 KB)            use counts of split row tiles (4095 ints) + the status word
 //   [16 KB, kGemvEnd)     tagged partial sums of the GEMV kernel, 8 KB per SM, room for 160 SMs
-//   then 40 KB of flags of the tensor-core GEMM (64 per CTA; zero between launches)
-//   then its fp32 partial tiles, one per CTA: room for 148 of 128 rows x 256 batch columns
+//   then the tensor-core GEMM's flags (48 per CTA, room for 160 CTAs) and its launch counter (64 bits)
+//   then its fp32 partial tiles, one per CTA of 128 rows x the batch tile: room for 148 of 256 columns,
+//   so for every CTA with the 192 columns that the batch tile has at most
 constexpr size_t kCounterBytes = 16384;
 constexpr int kStatusWord = 4095;
 constexpr size_t kGemvEnd = kCounterBytes + (size_t)160 * 1024 * sizeof(uint2);
 constexpr size_t kTcFlagsOffset = kGemvEnd;
-constexpr size_t kTcPartialOffset = kTcFlagsOffset + (size_t)160 * 64 * sizeof(int);
+constexpr int kTcFlagsPerRank = 48;  // (192 batch columns / 16) x (128 weight rows / 32)
+constexpr size_t kTcLaunchesOffset = kTcFlagsOffset + (size_t)160 * kTcFlagsPerRank * sizeof(int);
+constexpr size_t kTcPartialOffset = kTcLaunchesOffset + 256;
 constexpr size_t kTcPartialTileBytes = (size_t)128 * 256 * sizeof(float);
 constexpr size_t kWorkspaceBytes = kTcPartialOffset + 148 * kTcPartialTileBytes;
 

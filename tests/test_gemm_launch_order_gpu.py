@@ -106,3 +106,27 @@ def test_no_launch_reads_a_tiled_buffer_early_that_the_kernel_before_wrote(m):
     (repack,) = {a for a, _, _ in edges} - {b for _, b, _ in edges}  # the first kernel
     assert not any(programmatic for a, _, programmatic in edges if a == repack), edges
     assert any(programmatic for _, _, programmatic in edges), edges
+
+
+@pytest.mark.parametrize("left", [1, 2])
+def test_flags_of_an_earlier_launch_are_not_taken_for_this_ones(left):
+    """What a launch whose wait ran out can leave behind: flags published late, sums that belong to nothing, a status
+    word that is set.  Few tiles over long rows, so that nearly every CTA parks its sums; launches 1 and 2 on
+    the workspace are over."""
+    m, n, k = 40, 64, 64 * 150
+    layer = models.QuantisedLinear.create(torch.randn((n, k), device="cuda").bfloat16(), models.QuantisationConfig(4, 64))
+    x = torch.randn((m, k), device="cuda").bfloat16()
+    want = [layer(x) for _ in range(3)][-1]
+    workspace = native.workspace(x.device)
+    flags, counted, status = 1327104, 160 * 48 * 4, 4095 * 4  # as laid out in lut_table.cuh
+    assert bool((workspace[flags: flags + counted].view(torch.int32) != 0).any())
+    workspace[flags: flags + counted].view(torch.int32).fill_(left)
+    workspace[flags + counted + 256:].view(torch.float32).fill_(float("nan"))
+    workspace[status: status + 4].view(torch.int32).fill_(1)
+    try:
+        for _ in range(3):
+            assert torch.equal(layer(x), want)
+        assert native.device_status() == 1  # set until the workspace is initialised again
+    finally:
+        native.check(native.lib().fdk_workspace_init(workspace.data_ptr(), workspace.numel(), native._stream()))
+    assert torch.equal(layer(x), want) and native.device_status() == 0
