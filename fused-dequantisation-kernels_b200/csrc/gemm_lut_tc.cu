@@ -575,6 +575,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     // Second uses of a code slot or stage wait for MMAs, hence for x; the first ones do not, and fill
     // tensor memory while the kernel before is still running.
     auto wait_for_x = [&] { asm volatile("griddepcontrol.wait;" ::: "memory"); };
+    uint32_t held = 0;  // the barrier of the slot that the last fetch read, to be handed back
     auto fetch = [&](RowCodes<BITS>& codes, uint32_t& s2) -> int {
       while (u < u1) {
         const int nb = KSB == 1 ? 1 : blocks_of(ks);
@@ -586,9 +587,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           codes.load(slab + slab_off, jb, g, r, half, x);
           const uint32_t scw = ring32(slab + scale_off + jb * 128);
           s2 = half ? prmt<0x3232>(scw, 0u) : prmt<0x1010>(scw, 0u);
+          held = bar;
+        } else if (lane == 0) {
+          mbar_arrive(bar);
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar);
         const int block = KSB == 1 ? u - u0 : i + jb;
         if constexpr (KSB == 1) {
           u += kSets;
@@ -604,6 +606,15 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       }
       return -1;
     };
+    // Hands the slot back.  The copy that refills it writes through the async proxy, which a barrier arrival
+    // alone does not order after the reads above: they were still on their way (queued behind stores to
+    // tensor memory, with the tensor pipe busy) when the new codes came in, about once in a million blocks at
+    // 1000 rows of 22528 x 3072.
+    auto release = [&] {
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(held);
+    };
     // A block's stores to tensor memory are awaited and handed over while the lookups of the next
     // one are in flight, whose codes were fetched between the two halves of this one.
     auto hand_over = [&](int s) {
@@ -615,6 +626,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     RowCodes<BITS> codes;
     uint32_t s2 = 0;
     int block = fetch(codes, s2), stored = -1;
+    if (block >= 0) release();
     while (block >= 0) {
       const int s = block & (S - 1);
       uint32_t v[16];
@@ -629,6 +641,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       codes.template decode<3, FP16, WIDE>(lane_base, s2, v, 8);
       block = fetch(codes, s2);
       tmem_store16(a_lane + 32 * s + 16, v);
+      if (block >= 0) release();  // here, where the next lookups need the codes anyway
       stored = s;
     }
     if (stored >= 0 && !timed_out) hand_over(stored);

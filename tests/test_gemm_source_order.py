@@ -20,3 +20,9 @@ def test_partial_sums_are_read_after_every_lanes_acquire():
 def test_flags_are_published_after_every_lanes_stores():
     hand_over = between("if (begin != 0) {  // publish", "st.relaxed.gpu.global")
     assert 0 <= hand_over.index("__syncwarp();") < hand_over.index("__threadfence();")
+
+
+def test_code_slots_are_handed_back_behind_a_proxy_fence():
+    """Plain reads and the bulk copy that refills the slot go through different proxies."""
+    release = between("auto release = [&] {", "mbar_arrive(held)")
+    assert release.index("fence.proxy.async.shared::cta") < release.index("__syncwarp();")
