@@ -4,6 +4,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 
 #include "../../include/fdk_b200.h"
@@ -39,6 +40,21 @@ struct DeviceInfo {
 };
 // Cached per device; returns a status code.
 int device_info(DeviceInfo* out);
+
+// Lets a kernel without static shared memory use all that a block may have, once per device (`done`: one per
+// kernel).  The limit is the device's and not the call's: threads that meet here set the same value, in
+// whatever order.
+template <class Kernel>
+int allow_all_smem(Kernel kernel, std::atomic<bool> (&done)[64], const DeviceInfo& di) {
+  int dev = 0;
+  FDK_CUDA(cudaGetDevice(&dev));
+  std::atomic<bool>& have = done[dev & 63];
+  if (!have.load(std::memory_order_acquire)) {
+    FDK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, di.max_smem_optin));
+    have.store(true, std::memory_order_release);
+  }
+  return FDK_OK;
+}
 
 // ---- 16-bit float helpers --------------------------------------------------
 template <bool FP16>

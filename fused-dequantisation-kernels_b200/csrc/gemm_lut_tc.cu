@@ -669,13 +669,15 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
 int encode_fn(EncodeTiledFn* out) {
-  static EncodeTiledFn fn = nullptr;
+  static std::atomic<EncodeTiledFn> found{nullptr};
+  EncodeTiledFn fn = found.load(std::memory_order_acquire);
   if (fn == nullptr) {
     void* sym = nullptr;
     cudaDriverEntryPointQueryResult qres;
     FDK_CUDA(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &qres));
     FDK_CHECK_ARG(qres == cudaDriverEntryPointSuccess && sym != nullptr, FDK_ERR_CUDA, "cuTensorMapEncodeTiled not found");
     fn = (EncodeTiledFn)sym;
+    found.store(fn, std::memory_order_release);
   }
   *out = fn;
   return FDK_OK;
@@ -731,13 +733,8 @@ int launch_tc(TcParams p, const void* lut_host, const CUtensorMap& map, int grid
   const size_t smem = plan_tc_smem<BITS>(base, (uint32_t)di.max_smem_optin, p);
   FDK_CHECK_ARG(smem != 0, FDK_ERR_CUDA, "no shared-memory plan fits %d bytes", di.max_smem_optin);
   auto kernel = gemm_lut_tc_kernel<BITS, FP16>;
-  static size_t configured[64] = {};
-  int dev = 0;
-  FDK_CUDA(cudaGetDevice(&dev));
-  if (configured[dev & 63] < smem) {
-    FDK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured[dev & 63] = smem;
-  }
+  static std::atomic<bool> allowed[64] = {};
+  if (int st = allow_all_smem(kernel, allowed, di)) return st;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(kTcThreads);

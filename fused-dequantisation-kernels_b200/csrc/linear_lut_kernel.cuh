@@ -1058,17 +1058,12 @@ size_t plan_smem(uint32_t base, int warps, size_t limit, bool need_resident, Lin
   return layout(1, kXDirect);
 }
 
-// Sets the kernel's shared-memory limit once per device and launches it.
 template <class Kernel, int BITS>
-int launch_kernel(Kernel kernel, std::atomic<size_t> (&configured)[64], const LinearParams& p, const InlineLut<BITS>& inl,
+int launch_kernel(Kernel kernel, std::atomic<bool> (&allowed)[64], const LinearParams& p, const InlineLut<BITS>& inl,
                   int grid, int threads, size_t smem, unsigned flags, cudaStream_t stream) {
-  int dev = 0;
-  FDK_CUDA(cudaGetDevice(&dev));
-  std::atomic<size_t>& have = configured[dev & 63];
-  if (have.load(std::memory_order_acquire) < smem) {
-    FDK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    have.store(smem, std::memory_order_release);
-  }
+  DeviceInfo di;
+  if (int st = device_info(&di)) return st;
+  if (int st = allow_all_smem(kernel, allowed, di)) return st;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(threads);
@@ -1086,8 +1081,8 @@ int launch_kernel(Kernel kernel, std::atomic<size_t> (&configured)[64], const Li
 template <int BITS, int NB, int WARPS, bool FP16, int EPI, int XM, int NORM, bool TEAM>
 int launch_team(const LinearParams& p, const InlineLut<BITS>& inl, int grid, size_t smem, unsigned flags,
                 cudaStream_t stream) {
-  static std::atomic<size_t> configured[64] = {};
-  return launch_kernel(linear_lut_kernel<BITS, NB, WARPS, FP16, EPI, XM, NORM, TEAM>, configured, p, inl, grid,
+  static std::atomic<bool> allowed[64] = {};
+  return launch_kernel(linear_lut_kernel<BITS, NB, WARPS, FP16, EPI, XM, NORM, TEAM>, allowed, p, inl, grid,
                        (WARPS + 1) * 32, smem, flags, stream);
 }
 
