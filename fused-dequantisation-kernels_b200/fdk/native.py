@@ -296,16 +296,18 @@ _workspaces: dict[tuple[int, int], Tensor] = {}
 
 def workspace(device: torch.device) -> Tensor:
     """One zero-initialised scratch buffer per (device, stream).  Allocated on first use,
-    so the first call on a stream must happen before that stream is captured in a graph."""
+    so the first call on a stream must happen before that stream is captured in a graph.  The stream is
+    the one current on `device`, where the kernel will be launched, whichever device is current now."""
     index = device.index if device.index is not None else torch.cuda.current_device()
-    key = (index, _stream())
+    stream = torch._C._cuda_getCurrentRawStream(index)
+    key = (index, stream)
     ws = _workspaces.get(key)
     if ws is None:
         with torch.cuda.device(index):
             size = ctypes.c_size_t(0)
             check(lib().fdk_workspace_size(ctypes.byref(size)))
             ws = torch.empty(size.value, dtype=torch.uint8, device=f"cuda:{index}")
-            check(lib().fdk_workspace_init(ws.data_ptr(), size.value, _stream()))
+            check(lib().fdk_workspace_init(ws.data_ptr(), size.value, stream))
         _workspaces[key] = ws
     return ws
 
@@ -402,7 +404,7 @@ def prepare_linear_lut_host(tiled: Tensor, lut: Tensor, lut_bytes: bytes, x_dev:
     index = tiled.device.index
     fixed_a = (tiled.data_ptr(), lut.data_ptr(), lut_bytes)
     fixed_b = (m, n, k, bits, dtype_code(dtype), x_dev.data_ptr(), out_dev.data_ptr(), ws.data_ptr(), ws.numel(),
-               0 if synchronise else FLAG_NO_SYNC, _stream())
+               0 if synchronise else FLAG_NO_SYNC, torch._C._cuda_getCurrentRawStream(index))
     keep = (tiled, lut, x_dev, out_dev, ws)  # the buffers live as long as the call does
 
     def call(x_host_ptr: int, out_host_ptr: int, _keep=keep) -> None:
