@@ -749,12 +749,9 @@ int launch_tc(TcParams p, const void* lut_host, const CUtensorMap& map, int grid
   return FDK_OK;
 }
 
-}  // namespace
-
-// Batches above 16 rows.  Called by fdk_linear_lut.
-int gemm_lut_tc(const void* x, const void* tiled, const void* lut, const void* lut_host, void* out, int m, int n,
-                int k, int bits, bool fp16, void* workspace, size_t workspace_bytes, int sm_count, bool pdl,
-                cudaStream_t stream) {
+int gemm_rows(const void* x, const void* tiled, const void* lut, const void* lut_host, void* out, int m, int n,
+              int k, int bits, bool fp16, void* workspace, size_t workspace_bytes, int sm_count, bool pdl,
+              cudaStream_t stream) {
   EncodeTiledFn encode = nullptr;
   if (int st = encode_fn(&encode)) return st;
   const TiledDims d = tiled_dims(n, k, bits);
@@ -771,7 +768,6 @@ int gemm_lut_tc(const void* x, const void* tiled, const void* lut, const void* l
   p.k_blocks = k / kBlock;
   p.k_slabs = d.k_slabs;
   const long long tiles = (long long)((n + kTcTileRows - 1) / kTcTileRows) * p.m_tiles, units = tiles * d.k_slabs;
-  FDK_CHECK_ARG(units < (1ll << 31), FDK_ERR_SHAPE, "m=%d, n=%d, k=%d: too many tiles", m, n, k);
   p.tiles = (int)tiles;
   // eight A stages fit tensor memory beside two accumulators of 128 columns, four beside two of 192
   p.stages_log2 = p.n_tile <= 128 ? 3 : 2;
@@ -812,6 +808,26 @@ int gemm_lut_tc(const void* x, const void* tiled, const void* lut, const void* l
     case 4: return fp16 ? launch_tc<4, true>(p, lut_host, map, grid, pdl, stream) : launch_tc<4, false>(p, lut_host, map, grid, pdl, stream);
     default: return fp16 ? launch_tc<8, true>(p, lut_host, map, grid, pdl, stream) : launch_tc<8, false>(p, lut_host, map, grid, pdl, stream);
   }
+}
+
+}  // namespace
+
+// Batches above 16 rows.  Called by fdk_linear_lut.  One launch, unless its units, and steps beyond
+// them, would not fit 32 bits (100 thousand rows of 262080 x 65536): then one after another for as many whole
+// batch tiles as do.
+int gemm_lut_tc(const void* x, const void* tiled, const void* lut, const void* lut_host, void* out, int m, int n,
+                int k, int bits, bool fp16, void* workspace, size_t workspace_bytes, int sm_count, bool pdl,
+                cudaStream_t stream) {
+  const long long per_batch_tile = (long long)((n + kTcTileRows - 1) / kTcTileRows) * tiled_dims(n, k, bits).k_slabs;
+  const long long most = ((1ll << 30) / per_batch_tile) * kTcMaxBatch;
+  FDK_CHECK_ARG(most > 0, FDK_ERR_SHAPE, "n=%d, k=%d: too many slabs", n, k);
+  for (long long m0 = 0; m0 < m; m0 += most) {
+    const int rows = m - m0 < most ? (int)(m - m0) : (int)most;
+    if (int st = gemm_rows((const uint16_t*)x + (size_t)m0 * k, tiled, lut, lut_host, (uint16_t*)out + (size_t)m0 * n, rows, n, k,
+                           bits, fp16, workspace, workspace_bytes, sm_count, pdl, stream))
+      return st;
+  }
+  return FDK_OK;
 }
 
 }  // namespace fdk
