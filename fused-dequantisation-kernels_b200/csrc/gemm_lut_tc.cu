@@ -28,8 +28,8 @@
 // 12.0 us; 2048 rows of 28672 x 4096 791 -> 352 us (1.37 PFLOP/s).  Tried and not kept: groups
 // of four blocks per copy, barrier and stage (18.4 us at 32 rows of 8192^2 against 16.7: a set
 // then waits for a whole group, and the larger stages leave fewer of them).
-// Every wait is bounded; one that runs out sets a status bit, and the kernel still frees its
-// tensor memory and returns.  Under programmatic launch the bounds count this kernel's own time only: a
+// Every wait is bounded; one that runs out sets a status bit, and the kernel still lets copies and MMAs on
+// their way arrive, frees its tensor memory and returns.  Under programmatic launch the bounds count this kernel's own time only: a
 // role waits for the kernel before (griddepcontrol.wait, which has no bound) ahead of its first bounded
 // wait that x, and so that kernel, can hold up.
 #include <cuda.h>
@@ -650,7 +650,20 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   }
   if (timed_out && lane == 0) atomicOr(p.status, kTcStatusTimeout);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
+  if (__syncthreads_or(timed_out)) {
+    // A role gave up: copies and MMAs may still be on their way into shared and tensor memory, and their
+    // barriers no longer tell.  They take microseconds; the block keeps its memory for ten milliseconds.
+    if (threadIdx.x == 0) {
+      unsigned long long t0, now;
+      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+      for (uint32_t spin = 0; spin < (1u << 20); ++spin) {
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+        if (now - t0 > 10000000ull) break;
+        __nanosleep(1000);
+      }
+    }
+    __syncthreads();
+  }
   // Every CTA of a launch that cuts tiles has units, so this thread has waited for the launch before, and
   // every warp of the CTA has read the count.
   if (p.split && threadIdx.x == 0)
