@@ -77,3 +77,25 @@ def test_every_run_gives_the_same_bits(bits):
     for _ in range(500):
         differ += (layer(x) != first).any()
     assert differ.item() == 0 and native.device_status() == 0
+
+
+def test_room_for_some_partial_sums_only():
+    """A workspace for fewer CTAs than would share the tiles: they are not cut, and nothing is written behind it."""
+    m, n, k = 40, 300, 640
+    layer, x, want = problem(m, n, k, 4, torch.bfloat16)
+    slot, partial = 48 * 128 * 4, 16384 + 160 * 1024 * 8 + 160 * 48 * 4 + 256  # 48: the batch tile
+    for slots in (0, 1, 3, 160):
+        size = partial + slots * slot
+        buffer = torch.full((size + 4096,), 0xA5, device="cuda", dtype=torch.uint8)
+        native.check(native.lib().fdk_workspace_init(buffer.data_ptr(), size, native._stream()))
+        for _ in range(2):
+            out = torch.full((m, n), float("nan"), device="cuda", dtype=torch.bfloat16)
+            native.check(native.lib().fdk_linear_lut(
+                x.data_ptr(), layer.tiled().data_ptr(), layer.lut.data_ptr(), layer.lut_bytes(), out.data_ptr(), m, n, k, 4,
+                native.DTYPE_BF16, buffer.data_ptr(), size, 0, native._stream()))
+            check(out, want, torch.bfloat16)
+        word = ctypes.c_int(-1)
+        native.check(native.lib().fdk_workspace_status(buffer.data_ptr(), ctypes.byref(word)))
+        assert word.value == 0 and bool((buffer[size:] == 0xA5).all())
+        used = bool((buffer[partial:size] != 0).any())
+        assert used == (slots == 160)
