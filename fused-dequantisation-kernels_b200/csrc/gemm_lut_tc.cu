@@ -607,9 +607,12 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       return -1;
     };
     // Hands the slot back.  The copy that refills it writes through the async proxy, which a barrier arrival
-    // alone does not order after the reads above: they were still on their way (queued behind stores to
-    // tensor memory, with the tensor pipe busy) when the new codes came in, about once in a million blocks at
-    // 1000 rows of 22528 x 3072.
+    // alone does not order after the reads above: with an arrival right behind them they were still on
+    // their way (queued behind stores to tensor memory, with the tensor pipe busy) when the new codes came in,
+    // about once in a million blocks at 1000 rows of 22528 x 3072.  Hence the fence, and it stands behind the
+    // block's first store to tensor memory, which cannot issue before codes and scale are in registers: a fence
+    // right behind the reads waits for them (48 rows of 11264 x 3072 13.9 us against 12.5, 2048 of 28672 x 4096
+    // 362 against 344; where 128 batch rows leave a set one slot, 8192^2, 26.0 against 26.3).
     auto release = [&] {
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
@@ -626,7 +629,6 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     RowCodes<BITS> codes;
     uint32_t s2 = 0;
     int block = fetch(codes, s2), stored = -1;
-    if (block >= 0) release();
     while (block >= 0) {
       const int s = block & (S - 1);
       uint32_t v[16];
@@ -637,11 +639,11 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       if (!mbar_wait(empty + 8 * s, ((block >> p.stages_log2) & 1) ^ 1)) { timed_out = true; break; }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       tmem_store16(a_lane + 32 * s, v);
+      release();
       codes.template decode<2, FP16, WIDE>(lane_base, s2, v, 0);
       codes.template decode<3, FP16, WIDE>(lane_base, s2, v, 8);
       block = fetch(codes, s2);
       tmem_store16(a_lane + 32 * s + 16, v);
-      if (block >= 0) release();  // here, where the next lookups need the codes anyway
       stored = s;
     }
     if (stored >= 0 && !timed_out) hand_over(stored);

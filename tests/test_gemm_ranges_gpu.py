@@ -79,6 +79,18 @@ def test_every_run_gives_the_same_bits(bits):
     assert differ.item() == 0 and native.device_status() == 0
 
 
+@pytest.mark.parametrize("bits", [1, 2, 3, 4, 8])
+@pytest.mark.parametrize("k", [64, 128, 320])
+def test_long_ranges_of_short_slabs(k, bits):
+    """Many tiles of one to five blocks: slabs of several blocks that hold one, segments shorter than the rings."""
+    for m in (20, 128, 700):
+        layer, x, want = problem(m, 30000, k, bits, torch.bfloat16)
+        y = layer(x)
+        check(y, want, torch.bfloat16)
+        assert all(torch.equal(layer(x), y) for _ in range(5))
+    assert native.device_status() == 0
+
+
 def test_room_for_some_partial_sums_only():
     """A workspace for fewer CTAs than would share the tiles: they are not cut, and nothing is written behind it."""
     m, n, k = 40, 300, 640
