@@ -24,10 +24,11 @@
 // 110 to 190 cycles); above, the tensor pipe (2 N cycles a block).  A in tensor memory keeps both
 // the store of the tile and the MMA's reads of it out of shared memory, and its MMAs of
 // small N are faster (a block at N = 32 takes 68 cycles, 161 with A in shared memory).  Before (A in
-// shared memory, eight dequantising warps, a tile per CTA) and now, 4 bits: 48 rows of 11264 x 3072 23.1 ->
-// 12.0 us; 2048 rows of 28672 x 4096 791 -> 352 us (1.37 PFLOP/s).  Tried and not kept: groups
-// of four blocks per copy, barrier and stage (18.4 us at 32 rows of 8192^2 against 16.7: a set
-// then waits for a whole group, and the larger stages leave fewer of them).
+// shared memory, eight dequantising warps, a tile per CTA) and now, 4 bits, public call: 48 rows of
+// 11264 x 3072, four in a graph, 92.4 -> 52.0 us; 2048 rows of 28672 x 4096 792 -> 406 to 428 us, by the clock
+// (1.12 to 1.19 PFLOP/s).  Tried and not kept: groups of four blocks per copy, barrier and stage (18.4 us at
+// 32 rows of 8192^2 against 16.7, kernel alone: a set then waits for a whole group, and the larger
+// stages leave fewer of them).
 // Every wait is bounded; one that runs out sets a status bit, and the kernel still lets copies and MMAs on
 // their way arrive, frees its tensor memory and returns.  Under programmatic launch the bounds count this kernel's own time only: a
 // role waits for the kernel before (griddepcontrol.wait, which has no bound) ahead of its first bounded
@@ -51,8 +52,8 @@ constexpr int kTcXWarp = kTcWarps - 2, kTcMmaWarp = kTcWarps - 1, kTcFirstCodeWa
 constexpr int kTcThreads = 32 * kTcWarps;
 constexpr int kTcTileRows = 128;
 // Batch rows of a tile (MMA N, at most 256).  With 192 two accumulators and four A stages fit tensor memory,
-// so a tile's epilogue overlaps the next tile; with 256 it does not: 4 bits, 1000 rows of 5120 x 3072
-// 35.9 us against 30.8, 256 of 3072^2 20.9 / 13.6, 2048 of 28672 x 4096 366 / 352.  128: 31.4, 13.6, 388.
+// so a tile's epilogue overlaps the next tile; with 256 it does not: 4 bits, kernel alone, 1000 rows of
+// 5120 x 3072 35.9 us against 30.8, 256 of 3072^2 20.9 / 13.6, 2048 of 28672 x 4096 366 / 352.  128: 31.4, 13.6, 388.
 constexpr int kTcMaxBatch = 192;
 constexpr int kTcMaxStages = 8;
 constexpr int kTcMaxCodeSlots = 16;

@@ -169,8 +169,10 @@ static int linear_lut_impl(const void* x, const void* tiled, const void* lut, co
       p.max_len = fu->max_len;
     }
   }
-  // up to 16 rows the register path is the faster one (two n-tiles from 9 rows on: 19.5-21 us
-  // at 8192^2 against 29-30 us for the tensor-core kernel and 26 us for bf16 cuBLAS)
+  // Up to 16 rows the register path, for its arithmetic: it multiplies fp32 block sums by the scale, where the
+  // tensor-core kernel rounds every scaled weight to 16 bits.  It is not the faster one at most widths (8192^2,
+  // 16 rows here against 17 there, us: 4 bits 17.4 / 16.9, 3 bits 25.2 / 20.2, 2 bits 17.4 / 18.4, 1 bit
+  // 19.1 / 17.7, 8 bits 25.2 / 22.7; 8 rows at 4 bits 14.0).
   if (fu == nullptr && ex == nullptr && !(flags & FDK_FLAG_SILU_PAIRS) && m > 16) {
     return gemm_lut_tc(x, tiled, lut, lut_host, out, m, n, k, bits, dtype == FDK_DTYPE_F16, workspace, workspace_bytes,
                        di.sm_count, (flags & FDK_FLAG_PDL) != 0, (cudaStream_t)stream);

@@ -9,7 +9,7 @@
 // stores of a warp are contiguous and a scale block is a group of 2 to 32 lanes; kQuantBatch
 // octets per lane are loaded before the first is coded.
 // `QuantisedLinear.create` and the tiled copy, 11264 x 3072, 4 bits: 877 us as framework operations (a
-// dozen passes, four of them over 32- or 64-bit intermediates), 76 us with this kernel (host-bound).
+// dozen passes, four of them over 32- or 64-bit intermediates), 78 us with this kernel (host-bound).
 #include <type_traits>
 
 #include "fdk_common.cuh"

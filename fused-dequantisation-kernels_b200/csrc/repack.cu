@@ -197,7 +197,7 @@ __device__ __forceinline__ void dequant8(const uint8_t* src, const uint16_t* __r
 // before the first is decoded; the byte table is looked up in shared memory, replicated per lane
 // (lut_table.cuh: no bank conflicts), and the scale multiplies two elements per instruction.
 // 8192^2, 4 bits, bf16: 86.9 us before (one octet per thread at a time, table read element by
-// element from global memory), 33.2 us now = 5.1 TB/s of W and codes.
+// element from global memory), 35.0 us now = 4.9 TB/s of W and codes.
 // Rows are contiguous and whole octets and whole blocks, so octets and scales are counted
 // through the matrix: octet o has its codes at BITS * o and its scale at o / (block_size / 8).
 constexpr int kDequantThreads = 512;
