@@ -81,6 +81,7 @@ struct TcParams {
   int k_blocks, k_slabs;  // k / 64; slabs per 64-row tile
   int stages_log2, code_slots;
   int split;              // ranges may cut tiles
+  int base, rem;          // CTA `rank` owns `base + (rank < rem)` consecutive units (whole tiles where they are not cut)
   float* partial;         // [rank][n_tile][128] fp32 sums of a CTA that does not own its first tile
   int* flags;             // [rank][column sixteenth][row quarter] the launch that published
   unsigned long long* launches;  // launches on this workspace with cut tiles
@@ -261,8 +262,8 @@ struct RowCodes {
 
 // Unit range of CTA `rank`: units are (tile, slab) pairs, a tile's slabs consecutive.
 __device__ __forceinline__ int range_begin(const TcParams& p, int rank) {
-  return p.split ? (int)((long long)p.tiles * p.k_slabs * rank / gridDim.x)
-                 : p.k_slabs * (int)((long long)p.tiles * rank / gridDim.x);
+  const int begin = rank * p.base + min(rank, p.rem);
+  return p.split ? begin : p.k_slabs * begin;
 }
 
 // Position in the unit sequence.  Stepped, not divided out: the warps that issue copies and MMAs
@@ -316,26 +317,59 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   const int u0 = range_begin(p, rank), u1 = range_begin(p, rank + 1);
   bool timed_out = false;
 
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < S; ++s) {
-      mbar_init(full + 8 * s, 5);  // x has arrived, and the four warps of a set have stored A
-      mbar_init(empty + 8 * s, 1);
+  // Start-up, everything at once: the code producers set up their own barriers and request the first codes, the x
+  // producer sets up the others, the MMA warp allocates tensor memory, and all other warps fill the table.
+  // (One after another, with a CTA-wide barrier ahead of the copies and one behind the table: the first codes were
+  // there 2.6 us after the start of the CTA.)
+  const size_t tile_bytes = (size_t)p.k_slabs * L::kSlabBytes;  // one 64-row tile
+  // two producer warps, a slab each in turn: wait, expectation and two copies take one of them ~300 cycles
+  auto request_codes = [&](const Cursor& c, int slot) {
+    const uint8_t* src = p.tiled + 2 * c.nt * tile_bytes + (size_t)c.ks * L::kSlabBytes;
+    const bool second = 2 * c.nt + 1 < p.row_tiles;
+    const uint32_t bar = c_full + 8 * slot, dst = p.c_addr[slot];
+    if (elect_one()) {
+      mbar_expect(bar, (uint32_t)L::kSlabBytes * (second ? 2 : 1));
+      bulk_copy(dst, src, L::kSlabBytes, bar);
+      if (second) bulk_copy(dst + (uint32_t)L::kSlabBytes, src + tile_bytes, L::kSlabBytes, bar);
     }
-    for (int c = 0; c < p.code_slots; ++c) {
-      mbar_init(c_full + 8 * c, 1);
-      mbar_init(c_empty + 8 * c, KSB == 1 ? 4 : kTcDequantWarps);  // one set, or all
-    }
-    for (int a = 0; a < kTcAccumulators; ++a) {
-      mbar_init(acc_full + 8 * a, 1);
-      mbar_init(acc_empty + 8 * a, kTcEpilogueWarps);
-    }
-    mbar_init(acc_last, 2);  // the last MMAs, and the launch number in shared memory
+  };
+  const bool code_producer = warp >= kTcFirstCodeWarp && warp < kTcXWarp;
+  Cursor c(p, code_producer ? u0 + warp - kTcFirstCodeWarp : u0);  // the producers' position
+  auto init_fence = [] {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  }
-  __syncthreads();
-  // The copy producers are off; the others fill the table first.
-  if (warp < kTcFirstCodeWarp || warp == kTcMmaWarp) {
+    __syncwarp();
+  };
+  if (code_producer) {
+    const int first = warp - kTcFirstCodeWarp;
+    const int mine = first + kTcCodeWarps * lane;
+    if (mine < p.code_slots) {
+      mbar_init(c_full + 8 * mine, 1);
+      mbar_init(c_empty + 8 * mine, KSB == 1 ? 4 : kTcDequantWarps);  // one set, or all
+    }
+    init_fence();
+    for (int slot = first; slot < p.code_slots; slot += kTcCodeWarps) {  // the first use of every slot
+      if (u0 + slot < u1) request_codes(c, slot);
+      for (int i = 0; i < kTcCodeWarps; ++i) c.next(p);
+    }
+  } else if (warp == kTcXWarp) {
+    if (lane == 0) asm volatile("prefetch.tensormap [%0];" ::"l"(&x_map) : "memory");
+    if (lane < S) {
+      mbar_init(full + 8 * lane, 5);  // x has arrived, and the four warps of a set have stored A
+      mbar_init(empty + 8 * lane, 1);
+    }
+    if (lane < kTcAccumulators) {
+      mbar_init(acc_full + 8 * lane, 1);
+      mbar_init(acc_empty + 8 * lane, kTcEpilogueWarps);
+    }
+    if (lane == 31) mbar_init(acc_last, 2);  // the last MMAs, and the launch number in shared memory
+    init_fence();
+  } else {
+    if (warp == kTcMmaWarp) {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "r"((uint32_t)kTcTmemColumns)
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
     constexpr int kFillThreads = kTcThreads - 32 * (kTcCodeWarps + 1);
     const int tid = warp == kTcMmaWarp ? kFillThreads - 32 + lane : threadIdx.x;
     auto fill = [&](auto word) {
@@ -344,15 +378,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     };
     if (p.lut == nullptr) fill([&](int i) { return inl.w[i]; });
     else fill([&](int i) { return __ldg(reinterpret_cast<const uint32_t*>(p.lut) + i); });
-    if (warp == kTcMmaWarp) {
-      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "r"((uint32_t)kTcTmemColumns)
-                   : "memory");
-      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    asm volatile("bar.sync 1, %0;" ::"n"(kFillThreads) : "memory");
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   // All of tensor memory is allocated, so it starts at address 0; a constant keeps the MMAs' operands
   // in uniform registers.
   constexpr uint32_t tmem_base = 0;
@@ -450,35 +479,24 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 
   if (segments == 0) {
     // more CTAs than units
-  } else if (warp >= kTcFirstCodeWarp && warp < kTcXWarp) {
+  } else if (code_producer) {
     // ---------------- code producer ----------------
-    // two warps, a slab each in turn: wait, expectation and two copies take one of them ~300 cycles
     const int first = warp - kTcFirstCodeWarp;
-    int slot = first, phase = 0;
-    const size_t tile_bytes = (size_t)p.k_slabs * L::kSlabBytes;  // one 64-row tile
-    Cursor c(p, u0 + first);
-    for (int u = u0 + first; u < u1; u += kTcCodeWarps) {
-      const uint8_t* src = p.tiled + 2 * c.nt * tile_bytes + (size_t)c.ks * L::kSlabBytes;
-      const bool second = 2 * c.nt + 1 < p.row_tiles;
-      const uint32_t bar = c_full + 8 * slot, dst = p.c_addr[slot];
+    int slot = first, phase = 1;  // the first round is on its way
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // from here on a slot is freed by way of x
+    for (int u = u0 + first + p.code_slots; u < u1; u += kTcCodeWarps) {
       if (!mbar_wait(c_empty + 8 * slot, phase ^ 1)) { timed_out = true; break; }
-      if (elect_one()) {
-        mbar_expect(bar, (uint32_t)L::kSlabBytes * (second ? 2 : 1));
-        bulk_copy(dst, src, L::kSlabBytes, bar);
-        if (second) bulk_copy(dst + (uint32_t)L::kSlabBytes, src + tile_bytes, L::kSlabBytes, bar);
-      }
+      request_codes(c, slot);
       for (int i = 0; i < kTcCodeWarps; ++i) c.next(p);
       if ((slot += kTcCodeWarps) >= p.code_slots) {
         slot -= p.code_slots;
         phase ^= 1;
-        asm volatile("griddepcontrol.wait;" ::: "memory");  // from here on a slot is freed by way of x
       }
     }
   } else if (warp == kTcXWarp) {
     // ---------------- x producer ----------------
     asm volatile("griddepcontrol.wait;" ::: "memory");
     int i = 0;
-    Cursor c(p, u0);
     for (int u = u0; u < u1 && !timed_out; ++u, c.next(p)) {
       const int nb = blocks_of(c.ks);
       for (int jb = 0; jb < nb; ++jb, ++i) {
@@ -808,6 +826,8 @@ int gemm_rows(const void* x, const void* tiled, const void* lut, const void* lut
   }
   p.split = room >= (size_t)grid;
   if (!p.split && tiles < grid) grid = (int)tiles;
+  p.base = (int)((p.split ? units : tiles) / grid);
+  p.rem = (int)((p.split ? units : tiles) % grid);
   CUtensorMap map;
   const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)m};
   const cuuint64_t strides[1] = {(cuuint64_t)k * 2};
