@@ -65,9 +65,17 @@ extern "C" int fdk_workspace_status(const void* workspace, int* status_host) {
   return FDK_OK;
 }
 
+// From how many rows on the kernel for batches that share x (skinny_lut_kernel.cuh) is the faster one (up to 16 rows), us per
+// launch in a graph, linear_lut_kernel.cuh / that one: 4 bits, 2 rows, 8192^2 11.0 / 12.0, 3072^2 4.4 / 5.6; 3 rows 12.05 /
+// 12.06, 5.8 / 5.7; 2 bits, 3 rows 11.1 / 11.8, 6.4 / 5.9; 5 rows of 14336 x 4096 13.2 / 11.0; one row of 8192^2: 3 bits
+// 16.4 / 12.6, 1 bit 12.2 / 11.4, 8 bits 27.1 / 18.1.
+static int skinny_rows(int bits) { return bits == 4 ? 3 : bits == 2 ? 5 : 1; }
+
+// skinny_partial: kSkinnyPartialBytes of scratch that hold nothing else, or null (a workspace of an older size).
 static int linear_lut_impl(const void* x, const void* tiled, const void* lut, const void* lut_host, void* out,
                            int m, int n, int k, int bits, int dtype, void* workspace, size_t workspace_bytes,
-                           unsigned flags, const fdk_tp_exchange* ex, const fdk_linear_fusion* fu, void* stream) {
+                           void* skinny_partial, unsigned flags, const fdk_tp_exchange* ex, const fdk_linear_fusion* fu,
+                           void* stream) {
   FDK_CHECK_ARG(m > 0 && n > 0 && k > 0, FDK_ERR_BAD_ARG, "m=%d, n=%d, k=%d must be positive", m, n, k);
   FDK_CHECK_ARG(bits_supported(bits), FDK_ERR_SHAPE, "bits=%d not in {1,2,3,4,8}", bits);
   FDK_CHECK_ARG(k % kBlock == 0, FDK_ERR_SHAPE, "k=%d must be a multiple of 64", k);
@@ -169,13 +177,25 @@ static int linear_lut_impl(const void* x, const void* tiled, const void* lut, co
       p.max_len = fu->max_len;
     }
   }
-  // Up to 16 rows the register path, for its arithmetic: it multiplies fp32 block sums by the scale, where the
-  // tensor-core kernel rounds every scaled weight to 16 bits.  It is not the faster one at most widths (8192^2,
-  // 16 rows here against 17 there, us: 4 bits 17.4 / 16.9, 3 bits 25.2 / 20.2, 2 bits 17.4 / 18.4, 1 bit
-  // 19.1 / 17.7, 8 bits 25.2 / 22.7; 8 rows at 4 bits 14.0).
+  // Up to 16 rows the register paths, for their arithmetic: they multiply fp32 block sums by the scale, where the
+  // tensor-core kernel rounds every scaled weight to 16 bits.  They are the faster ones too (8192^2, 4 bits, us: 16 rows
+  // here 14.0, 17 rows there 16.1).
   if (fu == nullptr && ex == nullptr && !(flags & FDK_FLAG_SILU_PAIRS) && m > 16) {
     return gemm_lut_tc(x, tiled, lut, lut_host, out, m, n, k, bits, dtype == FDK_DTYPE_F16, workspace, workspace_bytes,
                        di.sm_count, (flags & FDK_FLAG_PDL) != 0, (cudaStream_t)stream);
+  }
+  if (skinny_partial != nullptr && !norm && m >= skinny_rows(bits) && m <= 16) {
+    p.m = m;
+    p.x = (const uint16_t*)x;
+    p.out = (uint16_t*)out;
+    p.partial = (uint2*)skinny_partial;
+    switch (bits) {
+      case 1: return launch_skinny_bits<1>(p, lut_host, grid, dtype, flags, (cudaStream_t)stream);
+      case 2: return launch_skinny_bits<2>(p, lut_host, grid, dtype, flags, (cudaStream_t)stream);
+      case 3: return launch_skinny_bits<3>(p, lut_host, grid, dtype, flags, (cudaStream_t)stream);
+      case 4: return launch_skinny_bits<4>(p, lut_host, grid, dtype, flags, (cudaStream_t)stream);
+      default: return launch_skinny_bits<8>(p, lut_host, grid, dtype, flags, (cudaStream_t)stream);
+    }
   }
   for (int m0 = 0; m0 < m; m0 += 16) {
     p.m = (m - m0) < 16 ? (m - m0) : 16;
@@ -194,12 +214,16 @@ static int linear_lut_impl(const void* x, const void* tiled, const void* lut, co
   return FDK_OK;
 }
 
+static void* skinny_part(void* workspace, size_t workspace_bytes) {
+  return workspace_bytes >= kWorkspaceBytes ? (uint8_t*)workspace + kSkinnyPartialOffset : nullptr;
+}
+
 extern "C" int fdk_linear_lut(const void* x, const void* tiled, const void* lut, const void* lut_host,
                               void* out, int m, int n, int k, int bits, int dtype, void* workspace,
                               size_t workspace_bytes, unsigned flags, void* stream) {
   FDK_CHECK_ARG(out != nullptr, FDK_ERR_BAD_ARG, "null pointer");
-  return linear_lut_impl(x, tiled, lut, lut_host, out, m, n, k, bits, dtype, workspace, workspace_bytes, flags,
-                         nullptr, nullptr, stream);
+  return linear_lut_impl(x, tiled, lut, lut_host, out, m, n, k, bits, dtype, workspace, workspace_bytes,
+                         skinny_part(workspace, workspace_bytes), flags, nullptr, nullptr, stream);
 }
 
 // fdk_linear_lut_host moves its few kilobytes of activations with a kernel of its own where it
@@ -272,7 +296,7 @@ extern "C" int fdk_linear_lut_host(const void* x_host, const void* tiled, const 
   // read by every CTA and does need its copy in device memory.
   void* out = out_mapped != nullptr ? out_mapped : out_dev;
   if (int st = linear_lut_impl(x_dev, tiled, lut, lut_host, out, m, n, k, bits, dtype, workspace, workspace_bytes,
-                               inner, nullptr, nullptr, stream)) {
+                               skinny_part(workspace, workspace_bytes), inner, nullptr, nullptr, stream)) {
     return st;
   }
   if (out_mapped == nullptr) FDK_CUDA(cudaMemcpyAsync(out_host, out_dev, out_bytes, cudaMemcpyDeviceToHost, s));
@@ -284,8 +308,8 @@ extern "C" int fdk_linear_lut_fused(const void* x, const void* tiled, const void
                                     int m, int n, int k, int bits, int dtype, void* workspace, size_t workspace_bytes,
                                     unsigned flags, const fdk_linear_fusion* fusion, void* stream) {
   FDK_CHECK_ARG(fusion != nullptr, FDK_ERR_BAD_ARG, "fusion is null");
-  return linear_lut_impl(x, tiled, lut, lut_host, out, m, n, k, bits, dtype, workspace, workspace_bytes, flags,
-                         nullptr, fusion, stream);
+  return linear_lut_impl(x, tiled, lut, lut_host, out, m, n, k, bits, dtype, workspace, workspace_bytes,
+                         skinny_part(workspace, workspace_bytes), flags, nullptr, fusion, stream);
 }
 
 extern "C" int fdk_linear_norm_fits(int m, int k, int bits, int* fits_host) {
@@ -305,8 +329,8 @@ extern "C" int fdk_linear_lut_push(const void* x, const void* tiled, const void*
                                    int n, int k, int bits, int dtype, void* workspace, size_t workspace_bytes,
                                    unsigned flags, const fdk_tp_exchange* ex, void* stream) {
   FDK_CHECK_ARG(ex != nullptr, FDK_ERR_BAD_ARG, "exchange is null");
-  return linear_lut_impl(x, tiled, lut, lut_host, nullptr, m, n, k, bits, dtype, workspace, workspace_bytes, flags,
-                         ex, nullptr, stream);
+  return linear_lut_impl(x, tiled, lut, lut_host, nullptr, m, n, k, bits, dtype, workspace, workspace_bytes,
+                         skinny_part(workspace, workspace_bytes), flags, ex, nullptr, stream);
 }
 
 // ---- entry point that allocates nothing ---------------------------------------------------
@@ -318,7 +342,8 @@ extern "C" int fdk_linear_lut_push(const void* x, const void* tiled, const void*
 // loads the library holds until the process exits.
 constexpr int kStaticMaxSms = 160;
 constexpr size_t kStaticScratchBytes = kCounterBytes + (size_t)kStaticMaxSms * 1024 * sizeof(uint2);  // 1,327,104
-static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
+// the scratch of every kernel, and behind it the skinny kernel's partial sums
+static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes + kSkinnyPartialBytes];
 
 // The array's address on the current device (looked up once per device; nothing is allocated).
 static int static_scratch(void** out) {
@@ -351,7 +376,9 @@ extern "C" int fdk_linear_lut_static(const void* x, const void* tiled, const voi
                 "this GPU has %d multiprocessors and needs %zu bytes of scratch; the built-in scratch holds %zu "
                 "(up to %d multiprocessors): use fdk_linear_lut with a caller-allocated workspace",
                 di.sm_count, need, kStaticScratchBytes, kStaticMaxSms);
-  return fdk_linear_lut(x, tiled, lut, lut_host, out, m, n, k, bits, dtype, scratch, kStaticScratchBytes, flags, stream);
+  FDK_CHECK_ARG(out != nullptr, FDK_ERR_BAD_ARG, "null pointer");
+  return linear_lut_impl(x, tiled, lut, lut_host, out, m, n, k, bits, dtype, scratch, kStaticScratchBytes,
+                         (uint8_t*)scratch + kStaticScratchBytes, flags, nullptr, nullptr, stream);
 }
 
 extern "C" int fdk_static_status(int* status_host) {

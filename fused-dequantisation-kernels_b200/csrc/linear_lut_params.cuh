@@ -67,12 +67,18 @@ struct LinearParams {
   uint2* peer_stage[8];     // staging words {two 16-bit outputs, tag} [2][tp][slot / 2] of each rank, as mapped here
   const uint32_t* seq;      // local count of reduces done so far = number of this push
   long long stage_slot;     // elements of one (half, rank) slot
+  int epilogue;             // (skinny kernel) what is done with finished sums
 };
 
 // Plans shared memory and launches; one explicit instantiation per code width, each in a
 // translation unit of its own so that they compile in parallel.
 template <int BITS>
 int launch_bits(const LinearParams& p, const void* lut_host, int grid, int dtype, unsigned flags, cudaStream_t stream);
+
+// The kernel for batches that share x (skinny_lut_kernel.cuh), 1 to 16 rows, every output but with the RMSNorm
+// applied to the input; p.partial must have kSkinnyPartialBytes.
+template <int BITS>
+int launch_skinny_bits(LinearParams p, const void* lut_host, int sm_count, int dtype, unsigned flags, cudaStream_t stream);
 
 // Whether the kernel's fused RMSNorm, which needs all of x in shared memory, can take x [m, k].
 template <int BITS>

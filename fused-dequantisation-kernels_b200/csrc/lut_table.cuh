@@ -239,6 +239,7 @@ __device__ __forceinline__ int ld_relaxed_s32(const int* p) {
 //   then the tensor-core GEMM's flags (48 per CTA, room for 160 CTAs) and its launch counter (64 bits)
 //   then its fp32 partial tiles, one per CTA of 128 rows x the batch tile: room for 148 of 256 columns,
 //   so for every CTA with the 192 columns that the batch tile has at most
+//   then the tagged partial sums of the skinny kernel, 128 rows x 16 per SM, room for 160 SMs
 constexpr size_t kCounterBytes = 16384;
 constexpr int kStatusWord = 4095;
 constexpr size_t kGemvEnd = kCounterBytes + (size_t)160 * 1024 * sizeof(uint2);
@@ -247,7 +248,9 @@ constexpr int kTcFlagsPerRank = 48;  // (192 batch columns / 16) x (128 weight r
 constexpr size_t kTcLaunchesOffset = kTcFlagsOffset + (size_t)160 * kTcFlagsPerRank * sizeof(int);
 constexpr size_t kTcPartialOffset = kTcLaunchesOffset + 256;
 constexpr size_t kTcPartialTileBytes = (size_t)128 * 256 * sizeof(float);
-constexpr size_t kWorkspaceBytes = kTcPartialOffset + 148 * kTcPartialTileBytes;
+constexpr size_t kSkinnyPartialOffset = kTcPartialOffset + 148 * kTcPartialTileBytes;
+constexpr size_t kSkinnyPartialBytes = (size_t)160 * 128 * 16 * sizeof(uint2);
+constexpr size_t kWorkspaceBytes = kSkinnyPartialOffset + kSkinnyPartialBytes;
 
 // Tensor-core GEMM for batches above 16 rows (gemm_lut_tc.cu).
 int gemm_lut_tc(const void* x, const void* tiled, const void* lut, const void* lut_host, void* out, int m, int n,

@@ -1,0 +1,5 @@
+#include "skinny_lut_kernel.cuh"
+
+namespace fdk {
+template int launch_skinny_bits<8>(LinearParams, const void*, int, int, unsigned, cudaStream_t);
+}  // namespace fdk
