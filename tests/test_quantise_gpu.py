@@ -36,6 +36,26 @@ def test_create_bytes_equal_torch(bits, n, k, block, dtype):
         assert got.lut.shape == want.lut.shape and got.scale.shape == want.scale.shape
 
 
+@pytest.mark.parametrize("bits,block", [(3, 64), (4, 128), (4, 32), (8, 64)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_large_matrices_equal_torch(bits, block, dtype):
+    """Sizes that look codes up in a table (4 M weights on, from 3 bits on), with every pattern among the weights,
+    codebooks in no order among them."""
+    n, k = 2101, 2048
+    gen = torch.Generator(device="cuda").manual_seed(bits + block)
+    w = (torch.randn((n, k), generator=gen, device="cuda") * k**-0.5).to(dtype)
+    patterns = torch.arange(65536, device="cuda", dtype=torch.int32).to(torch.int16).view(dtype)
+    w.view(-1)[-65536:] = torch.where(patterns.isfinite(), patterns, torch.zeros_like(patterns))
+    w[0, :7] = float("nan")
+    w[1, :7] = float("inf")
+    for lut in (torch.linspace(-1, 1, 2**bits, device="cuda").to(dtype), torch.randn(2**bits, generator=gen, device="cuda").to(dtype)):
+        config = models.QuantisationConfig(bits, block)
+        got, want = models.QuantisedLinear.create(w, config, lut=lut), by_torch(w, config, lut)
+        assert torch.equal(got.weight_data, want.weight_data)
+        assert torch.equal(got.scale.isnan(), want.scale.isnan())
+        assert torch.equal(got.scale.nan_to_num(), want.scale.nan_to_num())
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_every_quotient_class(dtype):
     """All 16-bit patterns as weights (subnormals, infinities and NaN among them), in blocks whose scales
