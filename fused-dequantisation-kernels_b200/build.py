@@ -3,15 +3,18 @@
     python fused-dequantisation-kernels_b200/build.py [--force]
 
 nvcc cross-compiles without a GPU.  Objects go to csrc/build/, the shared
-library to fdk/libfdk_b200.so; both are rebuilt only when a source is newer.
+library to fdk/libfdk_b200.so, the host side of eager calls (a Python extension in C++, without device
+code) to fdk/_eager.*.so; all are rebuilt only when a source is newer.
 """
 
 from __future__ import annotations
 
+import importlib.util
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -19,6 +22,7 @@ HERE = Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
 OBJ = CSRC / "build"
 LIB = HERE / "fdk" / "libfdk_b200.so"
+EAGER = HERE / "fdk" / ("_eager" + sysconfig.get_config_var("EXT_SUFFIX"))
 INCLUDE = HERE.parent / "include"
 
 NVCC_FLAGS = [
@@ -41,6 +45,21 @@ def _newest_header() -> float:
     return max(h.stat().st_mtime for h in headers)
 
 
+def _build_eager(force: bool, verbose: bool) -> None:
+    source, header = CSRC / "eager_calls.cpp", INCLUDE / "fdk_b200.h"
+    if not force and EAGER.exists() and EAGER.stat().st_mtime >= max(source.stat().st_mtime, header.stat().st_mtime):
+        return
+    torch = Path(importlib.util.find_spec("torch").origin).parent
+    cuda = Path(_nvcc()).resolve().parents[1]
+    include = [torch / "include", torch / "include/torch/csrc/api/include", cuda / "include", Path(sysconfig.get_paths()["include"])]
+    cmd = [shutil.which("g++") or "c++", "-O2", "-std=c++17", "-fPIC", "-shared", "-D_GLIBCXX_USE_CXX11_ABI=1",
+           *(f"-I{i}" for i in include), str(source), "-o", str(EAGER), f"-L{torch / 'lib'}",
+           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python"]
+    if verbose:
+        print(" ".join(cmd), file=sys.stderr)
+    subprocess.run(cmd, check=True)
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
     sources = sorted(CSRC.glob("*.cu"))
     OBJ.mkdir(exist_ok=True)
@@ -58,7 +77,9 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         return obj, stale
 
     with ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 1)) as pool:
+        eager = pool.submit(_build_eager, force, verbose)
         results = list(pool.map(compile_one, sources))
+        eager.result()
     objs = [o for o, _ in results]
     if force or any(s for _, s in results) or not LIB.exists():
         cmd = [nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-o", str(LIB), *map(str, objs)]

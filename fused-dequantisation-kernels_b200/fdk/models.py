@@ -65,14 +65,15 @@ class QuantisedLinear(nn.Module):
         kernel: Literal["triton", "torch.compile", "marlin", "marlin-lut"],
     ):
         super().__init__()
-        self.in_features = in_features
-        self.out_features = out_features
-        self.weight_data = nn.Parameter(weight_data, requires_grad=False)
-        self.scale = nn.Parameter(scale, requires_grad=False)
-        self.lut = nn.Buffer(lut)
-        self.kernel = kernel
-        self._tiled: Tensor | None = None  # derived from the three tensors above, never saved
-        self._tiled_key: tuple | None = None
+        # plain values straight into the instance's dictionary, where nn.Module's attribute assignment (over a microsecond
+        # each) puts them
+        self.__dict__.update(
+            in_features=in_features, out_features=out_features, kernel=kernel,
+            _tiled=None, _tiled_key=None,  # derived from the three tensors below, never saved
+        )
+        self.register_parameter("weight_data", nn.Parameter(weight_data, requires_grad=False))
+        self.register_parameter("scale", nn.Parameter(scale, requires_grad=False))
+        self.register_buffer("lut", nn.Buffer(lut))
 
     @property
     def bits(self) -> int:
@@ -103,6 +104,9 @@ class QuantisedLinear(nn.Module):
         return self._lut_host
 
     def forward(self, x: Tensor) -> Tensor:
+        out = native.eager_linear(self.__dict__, x)
+        if out is not None:
+            return out
         if x.ndim > 2:
             return self.forward(x.flatten(end_dim=-2)).unflatten(0, x.shape[:-1])
         if self.kernel == "torch.compile":
@@ -191,7 +195,7 @@ class QuantisedLinear(nn.Module):
             scale = None
             if c.bits <= 2:  # a mean depends on the order of its sum: the framework's own
                 scale = source.unflatten(-1, (-1, c.block_size)).abs().mean(dim=-1).clamp_min_(1e-12)
-            return cls(*weight.T.shape, *native.quantise(source, c.bits, c.block_size, lut, scale), kernel=c.kernel)
+            return cls(weight.shape[1], weight.shape[0], *native.quantise(source, c.bits, c.block_size, lut, scale), kernel=c.kernel)
         lut = nn.functional.pad(lut, (0, n_codes - lut.shape[0]), value=lut[-1])
 
         # one scale per block_size run of the input dimension

@@ -165,8 +165,30 @@ def lib() -> ctypes.CDLL:
                 continue  # optional entry points are bound where they are used
             fn.restype = restype
             fn.argtypes = argtypes
+        _bind_eager(handle)
         _lib = handle
     return _lib
+
+
+def _nothing(*args):
+    return None
+
+
+# The ordinary case of `QuantisedLinear.forward`, `quantise` and `repack` in one native call each (csrc/eager_calls.cpp);
+# None for every other case, which then takes the code here.
+eager_linear = eager_quantise = eager_repack = _nothing
+
+
+def _bind_eager(handle: ctypes.CDLL) -> None:
+    global eager_linear, eager_quantise, eager_repack
+    try:
+        from . import _eager
+    except ImportError:  # not built for this interpreter: the calls take longer
+        return
+    names = ("fdk_linear_lut", "fdk_quantise", "fdk_repack", "fdk_tiled_size")
+    if all(hasattr(handle, name) for name in names):
+        _eager.bind(*(ctypes.cast(getattr(handle, name), ctypes.c_void_p).value for name in names), _workspaces)
+        eager_linear, eager_quantise, eager_repack = _eager.linear, _eager.quantise, _eager.repack
 
 
 def check(status: int) -> None:
@@ -229,6 +251,9 @@ def can_quantise(weight: Tensor, bits: int, block_size: int, lut: Tensor) -> boo
 def quantise(weight: Tensor, bits: int, block_size: int, lut: Tensor, scale: Tensor | None) -> tuple[Tensor, Tensor, Tensor]:
     """Dense weight [n, k] and codebook -> packed codes, block scales, byte table (reference layout).
     The scales are the blocks' largest magnitudes, or those given."""
+    done = eager_quantise(weight, bits, block_size, lut, scale)
+    if done is not None:
+        return done
     _require_cuda(weight, lut)
     n, k = weight.shape
     dev, dt = weight.device, weight.dtype
@@ -249,6 +274,9 @@ def quantise(weight: Tensor, bits: int, block_size: int, lut: Tensor, scale: Ten
 
 def repack(codes: Tensor, scale: Tensor, n: int, k: int, bits: int, block_size: int) -> Tensor:
     """Packed codes + scales (reference layout) -> tiled uint8 buffer on the same device."""
+    tiled = eager_repack(codes, scale, n, k, bits, block_size)
+    if tiled is not None:
+        return tiled
     _require_cuda(codes, scale)
     assert codes.dtype == torch.uint8 and codes.is_contiguous() and scale.is_contiguous()
     tiled = torch.empty(tiled_size(n, k, bits), dtype=torch.uint8, device=codes.device)
