@@ -12,7 +12,7 @@
 //     load instruction, streaming loads that do not allocate in L1).  A warp holds two
 //     slabs of registers, used alternately: while it works on one, the loads of its next
 //     slab are in flight into the other, and L2 has been asked for the one after that
-//     (prefetch.global.L2, a line per lane).  The codes never pass through shared
+//     (one bulk request).  The codes never pass through shared
 //     memory.  The first loads are issued before the kernel waits for its predecessor
 //     on the stream (programmatic dependent launch): they read weights only.
 //   * Every warp reads the x fragments of its slab from L2 as it needs them (x is small and
@@ -184,7 +184,7 @@ __device__ __forceinline__ int cta_of(const LinearParams& p, int item) {
 // for two n-tiles): four CTAs' words of one 128-element group where a tile has one group (small
 // batches: several CTAs may share a tile), otherwise one CTA's words of four (eight) groups, so
 // that the number of trips does not grow with the batch.  A round that finds a stale tag is
-// repeated after a short sleep.  Returns false if that ran out.
+// repeated.  Returns false if that ran out.
 template <int NB>
 __device__ __forceinline__ bool fetch_foreign(const LinearParams& p, float* stash, int rt, uint32_t tag, int E) {
   constexpr int EMAX = 512 * NB;
@@ -214,7 +214,6 @@ __device__ __forceinline__ bool fetch_foreign(const LinearParams& p, float* stas
           ok = false;
           break;
         }
-        __nanosleep(64);
       }
 #pragma unroll
       for (int ci = 0; ci < 4; ++ci)
@@ -250,7 +249,6 @@ __device__ __forceinline__ bool fetch_foreign(const LinearParams& p, float* stas
           ok = false;
           break;
         }
-        __nanosleep(64);
       }
 #pragma unroll
       for (int gi = 0; gi < GROUPS; ++gi)
@@ -500,13 +498,22 @@ __device__ __forceinline__ uint4 ldg_l2(const void* p) {
   return v;
 }
 
-// Asks L2 for one whole slab, a 128-byte line per lane (a hint: no registers, no shared memory).
+// 32 bytes of x where `live`: lanes of unused batch columns read nothing (and keep lo and hi).
+__device__ __forceinline__ void ldg_l2_if(bool live, const void* p, uint4& lo, uint4& hi) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %9, 0;\n\t"
+      "@p ld.global.cg.v4.u32 {%0,%1,%2,%3}, [%8];\n\t"
+      "@p ld.global.cg.v4.u32 {%4,%5,%6,%7}, [%8+16];\n\t}"
+      : "+r"(lo.x), "+r"(lo.y), "+r"(lo.z), "+r"(lo.w), "+r"(hi.x), "+r"(hi.y), "+r"(hi.z), "+r"(hi.w)
+      : "l"(p), "r"((uint32_t)live)
+      : "memory");
+}
+
+// Asks L2 for one whole slab (a hint: no registers, no shared memory).  One bulk request instead of a
+// prefetch per line: those pass through the shared-memory pipe, which the lookups need, 17 wavefronts a slab.
 template <int BITS>
 __device__ __forceinline__ void prefetch_slab_l2(const uint8_t* slab, int lane) {
-  constexpr int kLines = Layout<BITS>::kSlabBytes / 128;
-#pragma unroll
-  for (int l = 0; l < kLines; l += 32)
-    if (l + lane < kLines) asm volatile("prefetch.global.L2 [%0];" ::"l"(slab + (l + lane) * 128));
+  if (lane == 0) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(slab), "n"(Layout<BITS>::kSlabBytes));
 }
 
 template <int BITS>
@@ -522,11 +529,11 @@ __device__ __forceinline__ void load_slab(SlabRegs<BITS>& s, const uint8_t* slab
   for (int jb = 0; jb < L::KSB; ++jb) s.sc[jb] = ldg_stream(sp + jb * 128);
 }
 
-// Spins (bounded, backing off) until *word == want.
+// Spins (bounded) until *word == want.  (Sleeps between the polls, here and in fetch_foreign, delayed what the launch ends
+// with: 5120 x 3072 5.25 us with them, 5.14 without.)
 __device__ __forceinline__ bool wait_shared_word(volatile int* word, int want) {
   for (uint32_t spins = 0; *word != want; ++spins) {
     if (spins > kSpinLimit) return false;
-    if (spins > 8) __nanosleep(32);
   }
   return true;
 }
@@ -556,7 +563,12 @@ __global__ void __launch_bounds__((WARPS + 1) * 32, 1)
   extern __shared__ __align__(128) uint8_t smem_raw[];
 
   const uint32_t raw = smem_addr(smem_raw);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // 4 bits: uniform for the compiler (positions and addresses of a warp then stay in uniform registers, and its branches are
+  // not taken for divergent ones), and the lanes of unused batch columns read no x: with one bulk prefetch per slab
+  // 8192^2 10.77 -> 10.2 us at one row, 128256 x 3072 50.2 -> 45.6.  At 2 bits both cost registers that the kernel does not
+  // have (10.0 -> 10.35).
+  constexpr bool LEAN = BITS == 4;
+  const int lane = threadIdx.x & 31, warp = LEAN ? __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0) : (int)threadIdx.x >> 5;
   const int g = lane >> 2, t = lane & 3;
   EpilogueSync* esync = reinterpret_cast<EpilogueSync*>(smem_raw);
   float* slots = reinterpret_cast<float*>(smem_raw + p.slots_off);
@@ -915,7 +927,7 @@ __global__ void __launch_bounds__((WARPS + 1) * 32, 1)
   uint32_t x_lane[NB];  // resident x: shared-memory address; otherwise: element offset into x
 #pragma unroll
   for (int nb = 0; nb < NB; ++nb) {
-    const int b = min(g + 8 * nb, p.m - 1);  // lanes of unused batch columns read a live row
+    const int b = min(g + 8 * nb, p.m - 1);  // lanes of unused batch columns point at a live row
     x_lane[nb] = XM == kXResident ? xres_addr + b * p.xres_row + t * 32 : (uint32_t)(b * p.k + t * 16);
   }
 
@@ -928,10 +940,12 @@ __global__ void __launch_bounds__((WARPS + 1) * 32, 1)
       uint32_t xb[NB][8];
 #pragma unroll
       for (int nb = 0; nb < NB; ++nb) {
-        uint4 lo, hi;
+        uint4 lo = make_uint4(0u, 0u, 0u, 0u), hi = lo;
         if constexpr (XM == kXResident) {
           lo = ring128(x_lane[nb] + col * 2);
           hi = ring128(x_lane[nb] + col * 2 + 16);
+        } else if constexpr (LEAN) {
+          ldg_l2_if(g + 8 * nb < p.m, p.x + x_lane[nb] + col, lo, hi);
         } else {
           lo = ldg_l2(p.x + x_lane[nb] + col);
           hi = ldg_l2(p.x + x_lane[nb] + col + 8);
