@@ -399,11 +399,21 @@ __global__ void silu_mul_kernel(const uint16_t* __restrict__ gate_up, uint16_t* 
     const uint32_t* uw = reinterpret_cast<const uint32_t*>(&uv);
     uint4 ov;
     uint32_t* ow = reinterpret_cast<uint32_t*>(&ov);
+    float gate[8], act[8];
+    bool exact = false;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      gate[j] = j & 1 ? pair_hi<false>(gw[j / 2]) : pair_lo<false>(gw[j / 2]);
+      exact = silu_quotient(gate[j], act[j]) || exact;
+    }
+    if (exact) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) act[j] = gate[j] / (1.f + __expf(-gate[j]));
+    }
+    auto rnd = [](float x) { return to_float<false>(from_float<false>(x)); };
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      auto act = [](float x) { return to_float<false>(from_float<false>(x / (1.f + __expf(-x)))); };
-      float a = act(pair_lo<false>(gw[j])) * pair_lo<false>(uw[j]);
-      float b = act(pair_hi<false>(gw[j])) * pair_hi<false>(uw[j]);
+      const float a = rnd(act[2 * j]) * pair_lo<false>(uw[j]), b = rnd(act[2 * j + 1]) * pair_hi<false>(uw[j]);
       ow[j] = (uint32_t)from_float<false>(a) | ((uint32_t)from_float<false>(b) << 16);
     }
     *reinterpret_cast<uint4*>(out + idx) = ov;

@@ -93,6 +93,17 @@ __device__ __forceinline__ float pair_hi(uint32_t w) {
   }
 }
 
+// x / (1 + e^-x) by the approximate reciprocal, and whether rounding it to bf16 might differ from rounding the quotient: the
+// product is within 3 units in the last place of it, so only where a rounding boundary of bf16 (half a unit is 0x8000 of
+// fp32's low half) lies within 8 units, or where the result is so small that the reciprocal or the product may
+// have been flushed.  The caller then divides.
+__device__ __forceinline__ bool silu_quotient(float x, float& q) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + __expf(-x)));
+  q = x * r;
+  return ((__float_as_uint(q) & 0xFFFFu) - (0x8000u - 8u)) <= 16u || !(fabsf(q) >= 1e-30f);
+}
+
 // ---- 3-bit helpers ----------------------------------------------------------
 // Source format for 3 bits: one MSB-first bit stream per row, element j at
 // stream bits [3j, 3j+3).  16 elements = 48 bits = 6 bytes.  The tiled buffer

@@ -164,7 +164,7 @@ __device__ __forceinline__ uint2 ring64(uint32_t addr) {
 
 // A lane's tile row and the code words of it.  The tiled buffer gives the 16 elements [16 t, 16 t + 16)
 // of rows 16 r + g and 16 r + g + 8 to lane 4 g + t; here lane 4 g + t collects the whole block of
-// ONE row, 8 t + g of the warp's 32, because a tensor-memory lane is a row of A.  Fetching piece c
+// ONE row, because a tensor-memory lane is a row of A (16 r + 8 half + g of a 64-row tile).  Fetching piece c
 // (16 elements) from all lanes at once would meet in a few banks, the rows being 64 and 512 bytes
 // apart, so lane l fetches piece c ^ x(l) in round c (x spreads what the bank bits of the row do
 // not) and the pieces are put in order by conditional swaps.
@@ -260,6 +260,14 @@ struct RowCodes {
   }
 };
 
+// 16-row sub-tile of a 64-row tile that lane 4 g + t of an even or odd quarter collects.  PAIRS: sub-tiles apart by two,
+// so that in a weight of alternating 32 gate rows and their 32 up rows both factors of an output are in one warp,
+// two lanes apart (the plain product keeps 32 consecutive rows together: its stores are 1 % of 2048 x 28672 faster for it).
+template <bool PAIRS>
+__device__ __forceinline__ int sub_tile_of(int quarter, int t) {
+  return PAIRS ? (quarter & 1) + 2 * (t >> 1) : 2 * (quarter & 1) + (t >> 1);
+}
+
 // Unit range of CTA `rank`: units are (tile, slab) pairs, a tile's slabs consecutive.
 __device__ __forceinline__ int range_begin(const TcParams& p, int rank) {
   const int begin = rank * p.base + min(rank, p.rem);
@@ -288,7 +296,9 @@ struct Cursor {
   }
 };
 
-template <int BITS, bool FP16>
+// SILU: out[m, n / 2] = silu(gate) * up of a weight whose rows alternate 32 gate rows and their 32 up rows, with the
+// roundings of the plain product followed by silu_mul_kernel.
+template <int BITS, bool FP16, bool SILU>
 __global__ void __launch_bounds__(kTcThreads, 1)
     gemm_lut_tc_kernel(const __grid_constant__ TcParams p, const __grid_constant__ InlineLut<BITS> inl,
                        const __grid_constant__ CUtensorMap x_map) {
@@ -392,7 +402,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   auto epilogue = [&](int tile, int begin, int end, uint32_t acc, int part, int parts, int launch) {
     const int nt = tile / p.m_tiles, mt = tile - nt * p.m_tiles;
     const int quarter = warp & 3;
-    const int row = nt * kTcTileRows + 32 * quarter + 8 * (lane & 3) + (lane >> 2);
+    const int row = nt * kTcTileRows + 64 * (quarter >> 1) + 16 * sub_tile_of<SILU>(quarter, lane & 3) + 8 * (lane & 1) + (lane >> 2);
     const size_t slot = (size_t)p.n_tile * kTcTileRows;
     const uint32_t taddr = acc + ((uint32_t)(quarter * 32) << 16);
     const int tile_end = (tile + 1) * p.k_slabs;
@@ -449,8 +459,33 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             }
           }
         }
-        if (row < p.n) {
-          const int b0 = mt * p.n_tile + c0;
+        const int b0 = mt * p.n_tile + c0;
+        if constexpr (SILU) {
+          // a gate lane takes the even columns and the up lane two lanes on the odd ones; each sends the other its factor
+          auto rnd = [](float x) { return to_float<FP16>(from_float<FP16>(x)); };
+          const bool is_up = (lane & 2) != 0;
+          const int width = p.n / 2;
+          float gate[8], up[8], act[8];
+          bool exact = false;  // some quotient has to be a division (silu_quotient)
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float own = rnd(is_up ? v[2 * j + 1] : v[2 * j]);
+            const float other = __shfl_xor_sync(0xffffffffu, rnd(is_up ? v[2 * j] : v[2 * j + 1]), 2);
+            gate[j] = is_up ? other : own;
+            up[j] = is_up ? own : other;
+            exact = silu_quotient(gate[j], act[j]) || exact;
+          }
+          if (exact) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) act[j] = gate[j] / (1.f + __expf(-gate[j]));
+          }
+          uint16_t* dst = p.out + (size_t)(b0 + is_up) * width + (nt * 2 + (quarter >> 1)) * 32 + 16 * (quarter & 1) + 8 * (lane & 1) + (lane >> 2);
+          if (row < p.n) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              if (b0 + 2 * j + is_up < p.m) dst[(size_t)(2 * j) * width] = from_float<FP16>(rnd(act[j]) * up[j]);
+          }
+        } else if (row < p.n) {
           uint16_t* dst = p.out + (size_t)b0 * p.n + row;
 #pragma unroll
           for (int j = 0; j < 16; ++j)
@@ -578,7 +613,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     // ---------------- dequantise ----------------
     const int set = warp >> 2, quarter = warp & 3;
     const int g = lane >> 2, t = lane & 3;
-    const int r = 2 * (quarter & 1) + (t >> 1), half = t & 1;  // the lane's row: 32 quarter + 8 t + g
+    const int r = sub_tile_of<SILU>(quarter, t), half = t & 1;  // the lane's row: 16 r + 8 half + g of its 64-row tile
     const int x = RowCodes<BITS>::first_piece(g, t);
     const uint32_t slab_off = (quarter >> 1) * (uint32_t)L::kSlabBytes;
     const uint32_t scale_off = slab_off + L::kCodeBytes + g * 16 + r * 4;
@@ -751,7 +786,7 @@ size_t plan_tc_smem(uint32_t base, uint32_t limit, TcParams& p) {
   return p.code_slots >= 4 ? used - base : 0;
 }
 
-template <int BITS, bool FP16>
+template <int BITS, bool FP16, bool SILU>
 int launch_tc(TcParams p, const void* lut_host, const CUtensorMap& map, int grid, bool pdl, cudaStream_t stream) {
   InlineLut<BITS> inl;
   if (lut_host != nullptr) {
@@ -766,7 +801,7 @@ int launch_tc(TcParams p, const void* lut_host, const CUtensorMap& map, int grid
   if (int st = device_info(&di)) return st;
   const size_t smem = plan_tc_smem<BITS>(base, (uint32_t)di.max_smem_optin, p);
   FDK_CHECK_ARG(smem != 0, FDK_ERR_CUDA, "no shared-memory plan fits %d bytes", di.max_smem_optin);
-  auto kernel = gemm_lut_tc_kernel<BITS, FP16>;
+  auto kernel = gemm_lut_tc_kernel<BITS, FP16, SILU>;
   static std::atomic<bool> allowed[64] = {};
   if (int st = allow_all_smem(kernel, allowed, di)) return st;
   cudaLaunchConfig_t cfg = {};
@@ -784,7 +819,7 @@ int launch_tc(TcParams p, const void* lut_host, const CUtensorMap& map, int grid
 }
 
 int gemm_rows(const void* x, const void* tiled, const void* lut, const void* lut_host, void* out, int m, int n,
-              int k, int bits, bool fp16, void* workspace, size_t workspace_bytes, int sm_count, bool pdl,
+              int k, int bits, bool fp16, bool silu, void* workspace, size_t workspace_bytes, int sm_count, bool pdl,
               cudaStream_t stream) {
   EncodeTiledFn encode = nullptr;
   if (int st = encode_fn(&encode)) return st;
@@ -837,30 +872,36 @@ int gemm_rows(const void* x, const void* tiled, const void* lut, const void* lut
                       strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                       CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   FDK_CHECK_ARG(r == CUDA_SUCCESS, FDK_ERR_CUDA, "cuTensorMapEncodeTiled failed with %d", (int)r);
+  auto launch = [&](auto bits_c) {
+    constexpr int BITS = decltype(bits_c)::value;
+    if (silu) return launch_tc<BITS, false, true>(p, lut_host, map, grid, pdl, stream);
+    return fp16 ? launch_tc<BITS, true, false>(p, lut_host, map, grid, pdl, stream)
+                : launch_tc<BITS, false, false>(p, lut_host, map, grid, pdl, stream);
+  };
   switch (bits) {
-    case 1: return fp16 ? launch_tc<1, true>(p, lut_host, map, grid, pdl, stream) : launch_tc<1, false>(p, lut_host, map, grid, pdl, stream);
-    case 2: return fp16 ? launch_tc<2, true>(p, lut_host, map, grid, pdl, stream) : launch_tc<2, false>(p, lut_host, map, grid, pdl, stream);
-    case 3: return fp16 ? launch_tc<3, true>(p, lut_host, map, grid, pdl, stream) : launch_tc<3, false>(p, lut_host, map, grid, pdl, stream);
-    case 4: return fp16 ? launch_tc<4, true>(p, lut_host, map, grid, pdl, stream) : launch_tc<4, false>(p, lut_host, map, grid, pdl, stream);
-    default: return fp16 ? launch_tc<8, true>(p, lut_host, map, grid, pdl, stream) : launch_tc<8, false>(p, lut_host, map, grid, pdl, stream);
+    case 1: return launch(std::integral_constant<int, 1>{});
+    case 2: return launch(std::integral_constant<int, 2>{});
+    case 3: return launch(std::integral_constant<int, 3>{});
+    case 4: return launch(std::integral_constant<int, 4>{});
+    default: return launch(std::integral_constant<int, 8>{});
   }
 }
 
 }  // namespace
 
-// Batches above 16 rows.  Called by fdk_linear_lut.  One launch, unless its units, and steps beyond
+// Batches above 16 rows.  Called by fdk_linear_lut and fdk_linear_lut_silu (silu: bf16, n a multiple of 64).  One launch, unless its units, and steps beyond
 // them, would not fit 32 bits (100 thousand rows of 262080 x 65536): then one after another for as many whole
 // batch tiles as do.
 int gemm_lut_tc(const void* x, const void* tiled, const void* lut, const void* lut_host, void* out, int m, int n,
-                int k, int bits, bool fp16, void* workspace, size_t workspace_bytes, int sm_count, bool pdl,
+                int k, int bits, bool fp16, bool silu, void* workspace, size_t workspace_bytes, int sm_count, bool pdl,
                 cudaStream_t stream) {
   const long long per_batch_tile = (long long)((n + kTcTileRows - 1) / kTcTileRows) * tiled_dims(n, k, bits).k_slabs;
   const long long most = ((1ll << 30) / per_batch_tile) * kTcMaxBatch;
   FDK_CHECK_ARG(most > 0, FDK_ERR_SHAPE, "n=%d, k=%d: too many slabs", n, k);
   for (long long m0 = 0; m0 < m; m0 += most) {
     const int rows = m - m0 < most ? (int)(m - m0) : (int)most;
-    if (int st = gemm_rows((const uint16_t*)x + (size_t)m0 * k, tiled, lut, lut_host, (uint16_t*)out + (size_t)m0 * n, rows, n, k,
-                           bits, fp16, workspace, workspace_bytes, sm_count, pdl, stream))
+    if (int st = gemm_rows((const uint16_t*)x + (size_t)m0 * k, tiled, lut, lut_host, (uint16_t*)out + (size_t)m0 * (silu ? n / 2 : n),
+                           rows, n, k, bits, fp16, silu, workspace, workspace_bytes, sm_count, pdl, stream))
       return st;
   }
   return FDK_OK;

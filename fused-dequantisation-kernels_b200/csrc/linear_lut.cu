@@ -181,7 +181,7 @@ static int linear_lut_impl(const void* x, const void* tiled, const void* lut, co
   // tensor-core kernel rounds every scaled weight to 16 bits.  They are the faster ones too (8192^2, 4 bits, us: 16 rows
   // here 14.0, 17 rows there 16.1).
   if (fu == nullptr && ex == nullptr && !(flags & FDK_FLAG_SILU_PAIRS) && m > 16) {
-    return gemm_lut_tc(x, tiled, lut, lut_host, out, m, n, k, bits, dtype == FDK_DTYPE_F16, workspace, workspace_bytes,
+    return gemm_lut_tc(x, tiled, lut, lut_host, out, m, n, k, bits, dtype == FDK_DTYPE_F16, false, workspace, workspace_bytes,
                        di.sm_count, (flags & FDK_FLAG_PDL) != 0, (cudaStream_t)stream);
   }
   if (skinny_partial != nullptr && !norm && m >= skinny_rows(bits) && m <= 16) {
@@ -224,6 +224,34 @@ extern "C" int fdk_linear_lut(const void* x, const void* tiled, const void* lut,
   FDK_CHECK_ARG(out != nullptr, FDK_ERR_BAD_ARG, "null pointer");
   return linear_lut_impl(x, tiled, lut, lut_host, out, m, n, k, bits, dtype, workspace, workspace_bytes,
                          skinny_part(workspace, workspace_bytes), flags, nullptr, nullptr, stream);
+}
+
+extern "C" int fdk_linear_lut_silu(const void* x, const void* tiled, const void* lut, const void* lut_host, void* out, int m, int n,
+                                   int k, int bits, void* workspace, size_t workspace_bytes, unsigned flags, void* stream) {
+  FDK_CHECK_ARG((flags & ~FDK_FLAG_PDL) == 0, FDK_ERR_BAD_ARG, "unknown flags 0x%x", flags);
+  if (m <= 16) {
+    return fdk_linear_lut(x, tiled, lut, lut_host, out, m, n, k, bits, FDK_DTYPE_BF16, workspace, workspace_bytes,
+                          flags | FDK_FLAG_SILU_PAIRS, stream);
+  }
+  // the checks of linear_lut_impl
+  FDK_CHECK_ARG(x && tiled && (lut || lut_host) && out, FDK_ERR_BAD_ARG, "null pointer");
+  FDK_CHECK_ARG(n > 0 && k > 0, FDK_ERR_BAD_ARG, "n=%d, k=%d must be positive", n, k);
+  FDK_CHECK_ARG(bits_supported(bits), FDK_ERR_SHAPE, "bits=%d not in {1,2,3,4,8}", bits);
+  FDK_CHECK_ARG(k % kBlock == 0 && n % kTileRows == 0, FDK_ERR_SHAPE, "n=%d and k=%d must be multiples of 64", n, k);
+  FDK_CHECK_ARG(((uintptr_t)x & 15) == 0 && ((uintptr_t)tiled & 15) == 0 && ((uintptr_t)lut & 15) == 0 && ((uintptr_t)out & 1) == 0,
+                FDK_ERR_ALIGN, "x, tiled and lut must be 16-byte aligned");
+  DeviceInfo di;
+  if (int st = device_info(&di)) return st;
+  FDK_CHECK_ARG(di.cc_major == 10, FDK_ERR_ARCH, "device has compute capability %d.%d", di.cc_major, di.cc_minor);
+  const TiledDims d = tiled_dims(n, k, bits);
+  FDK_CHECK_ARG(d.row_tiles < kStatusWord && (uint64_t)d.row_tiles * d.k_slabs * d.k_slabs < ((uint64_t)1 << 32), FDK_ERR_SHAPE,
+                "matrix of %d x %d slabs is too large", d.row_tiles, d.k_slabs);
+  FDK_CHECK_ARG(di.sm_count <= 160, FDK_ERR_ARCH, "%d multiprocessors: the workspace layout provides for 160", di.sm_count);
+  const size_t need = kCounterBytes + (size_t)di.sm_count * 1024 * sizeof(uint2);
+  FDK_CHECK_ARG(workspace != nullptr && workspace_bytes >= need && ((uintptr_t)workspace & 15) == 0, FDK_ERR_WORKSPACE,
+                "workspace must be a 16-byte aligned buffer of at least %zu bytes", need);
+  return gemm_lut_tc(x, tiled, lut, lut_host, out, m, n, k, bits, false, true, workspace, workspace_bytes, di.sm_count,
+                     (flags & FDK_FLAG_PDL) != 0, (cudaStream_t)stream);
 }
 
 // fdk_linear_lut_host moves its few kilobytes of activations with a kernel of its own where it

@@ -254,7 +254,7 @@ constexpr size_t kWorkspaceBytes = kSkinnyPartialOffset + kSkinnyPartialBytes;
 
 // Tensor-core GEMM for batches above 16 rows (gemm_lut_tc.cu).
 int gemm_lut_tc(const void* x, const void* tiled, const void* lut, const void* lut_host, void* out, int m, int n,
-                int k, int bits, bool fp16, void* workspace, size_t workspace_bytes, int sm_count, bool pdl,
+                int k, int bits, bool fp16, bool silu, void* workspace, size_t workspace_bytes, int sm_count, bool pdl,
                 cudaStream_t stream);
 
 // The dynamic shared memory address seen by kernels without static shared memory, asked of

@@ -152,12 +152,19 @@ class QuantisedLinear(nn.Module):
 
     def forward_silu_pairs(self, x: Tensor, out: Tensor) -> None:
         """For a fused gate|up projection whose rows alternate 32 gate rows and their 32 up rows:
-        out[m, n / 2] = silu(gate) * up, in the projection kernel itself up to 16 rows."""
+        out[m, n / 2] = silu(gate) * up, in the projection kernel itself."""
         assert x.ndim == 2 and self.out_features % 64 == 0
         if self.kernel != "torch.compile" and x.shape[0] <= 16:
             native.linear_lut(
                 x.contiguous(), self.tiled(), self.lut, out, self.out_features, self.in_features, self.bits,
                 pdl=True, lut_bytes=self.lut_bytes(), silu_pairs=True,
+            )
+        elif (
+            self.kernel != "torch.compile" and x.dtype == out.dtype == self.lut.dtype == torch.bfloat16 and out.is_contiguous()
+            and out.shape == (x.shape[0], self.out_features // 2)
+        ):
+            native.linear_lut_silu(
+                x.contiguous(), self.tiled(), self.lut, out, self.out_features, self.in_features, self.bits, self.lut_bytes(),
             )
         else:
             native.silu_mul(self.forward(x), out, group=32)

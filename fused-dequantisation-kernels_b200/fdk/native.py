@@ -134,6 +134,10 @@ _SIGNATURES = {
         ctypes.c_int,
         [ctypes.c_void_p] * 5 + [ctypes.c_int] * 5 + [ctypes.c_void_p, ctypes.c_size_t, ctypes.c_uint, ctypes.c_void_p],
     ),
+    "fdk_linear_lut_silu": (
+        ctypes.c_int,
+        [ctypes.c_void_p] * 5 + [ctypes.c_int] * 4 + [ctypes.c_void_p, ctypes.c_size_t, ctypes.c_uint, ctypes.c_void_p],
+    ),
     "fdk_linear_lut_host": (
         ctypes.c_int,
         [ctypes.c_void_p] * 5 + [ctypes.c_int] * 5
@@ -396,6 +400,19 @@ def linear_lut(
         )
     if status != OK:
         check(status)
+
+
+def linear_lut_silu(x: Tensor, tiled: Tensor, lut: Tensor, out: Tensor, n: int, k: int, bits: int, lut_bytes: bytes) -> None:
+    """out[m, n / 2] = silu(gate) * up of x [m, k] (bf16) with a weight whose rows alternate 32 gate rows and their 32 up rows."""
+    _require_cuda(x, tiled, lut, out)
+    ws = workspace(x.device)
+    with _on(x.device):
+        check(
+            lib().fdk_linear_lut_silu(
+                x.data_ptr(), tiled.data_ptr(), lut.data_ptr(), lut_bytes, out.data_ptr(), x.shape[0], n, k, bits,
+                ws.data_ptr(), ws.numel(), FLAG_PDL, _stream(),
+            )
+        )
 
 
 def linear_lut_host(
