@@ -151,6 +151,15 @@ __device__ __forceinline__ void tmem_load16(uint32_t addr, uint32_t (&v)[16]) {
       : "memory");
 }
 
+__device__ __forceinline__ void tmem_load8(uint32_t addr, uint32_t (&v)[8]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+      : "r"(addr)
+      : "memory");
+}
+
 __device__ __forceinline__ uint32_t ring32(uint32_t addr) {
   uint32_t v;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
@@ -411,6 +420,58 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       while (range_begin(p, last_rank + 1) < tile_end) ++last_rank;
     // flag of 16 columns of 32 rows: one warp publishes them, one consumes them
     auto flag = [&](int of_rank, int c0) { return p.flags + of_rank * kTcFlagsPerRank + (c0 >> 4) * 4 + quarter; };
+    auto await_shares = [&](int c0) {
+      for (int o = rank + 1 + lane; o <= last_rank; o += 32) {  // a lane per share
+        int* const f = flag(o, c0);
+        unsigned long long t0 = 0;
+        for (uint32_t spin = 0;; ++spin) {
+          int set;
+          asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(set) : "l"(f) : "memory");
+          if (set == launch) break;
+          if ((spin & 255u) == 255u) {
+            unsigned long long now;
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+            if (t0 == 0) t0 = now;
+            else if (now - t0 > 2000000000ull) { timed_out = true; break; }
+          }
+        }
+      }
+      timed_out = __any_sync(0xffffffffu, timed_out);
+      __syncwarp();  // the lanes' reads below come after every polling lane's acquire (a vote orders no memory)
+    };
+    // Several shares of a tile of few columns: eight columns at a time, so that every warp has some and the loads of four
+    // shares are in flight (32 rows: 5120 x 3072 8.97 us -> 8.58, 256 x 20480 11.2 -> 9.7; with one share, or with so many
+    // columns that the warps go round twice, 16 at a time are better: 48 rows of 11264 x 3072 11.8 against 12.6).
+    if (!SILU && last_rank > rank + 1 && p.n_tile <= 8 * parts) {
+      for (int c0 = 8 * part; c0 < p.n_tile; c0 += 8 * parts) {
+        uint32_t acc8[8];
+        tmem_load8(taddr + (uint32_t)c0, acc8);
+        float v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(acc8[j]);
+        await_shares(c0);
+        for (int o = rank + 1; o <= last_rank; o += 4) {  // in rank order
+          const float* theirs = p.partial + o * slot + (size_t)c0 * kTcTileRows + 32 * quarter + lane;
+          float t[4][8];
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) t[q][j] = o + q <= last_rank ? __ldcg(theirs + q * slot + j * kTcTileRows) : 0.f;
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] += t[q][j];
+        }
+        const int b0 = mt * p.n_tile + c0;
+        if (row < p.n) {
+          uint16_t* dst = p.out + (size_t)b0 * p.n + row;
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            if (b0 + j < p.m) dst[(size_t)j * p.n] = from_float<FP16>(v[j]);
+        }
+      }
+      return;
+    }
     for (int c0 = 16 * part; c0 < p.n_tile; c0 += 16 * parts) {
       uint32_t acc16[16];
       tmem_load16(taddr + (uint32_t)c0, acc16);
@@ -424,23 +485,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 #pragma unroll
         for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(acc16[j]);
         if (last_rank > rank) {
-          for (int o = rank + 1 + lane; o <= last_rank; o += 32) {  // a lane per share
-            int* const f = flag(o, c0);
-            unsigned long long t0 = 0;
-            for (uint32_t spin = 0;; ++spin) {
-              int set;
-              asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(set) : "l"(f) : "memory");
-              if (set == launch) break;
-              if ((spin & 255u) == 255u) {
-                unsigned long long now;
-                asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
-                if (t0 == 0) t0 = now;
-                else if (now - t0 > 2000000000ull) { timed_out = true; break; }
-              }
-            }
-          }
-          timed_out = __any_sync(0xffffffffu, timed_out);
-          __syncwarp();  // the lanes' reads below come after every polling lane's acquire (a vote orders no memory)
+          await_shares(c0);
           // in rank order; two shares' loads are in flight at a time
           for (int o = rank + 1; o <= last_rank; o += 2) {
             const float* theirs = p.partial + o * slot + at;
@@ -799,7 +844,15 @@ int launch_tc(TcParams p, const void* lut_host, const CUtensorMap& map, int grid
   if (int st = dynamic_smem_base(&base)) return st;
   DeviceInfo di;
   if (int st = device_info(&di)) return st;
-  const size_t smem = plan_tc_smem<BITS>(base, (uint32_t)di.max_smem_optin, p);
+  size_t smem = plan_tc_smem<BITS>(base, (uint32_t)di.max_smem_optin, p);
+  // 4 bits: eight stages of 128 batch rows leave four code slots, one a set, which then waits for every copy; with four
+  // stages there are sixteen (128 rows of 8192^2 24.8 us -> 21.75, of 3072^2 12.9 -> 11.8).  Eight slots beside
+  // eight stages of 112 rows are better than that (20.0 against 20.95), and so are the four at 8 bits, whose blocks take
+  // twice as long (27.2 against 28.1).
+  if (BITS == 4 && p.stages_log2 == 3 && p.code_slots < 8) {
+    p.stages_log2 = 2;
+    smem = plan_tc_smem<BITS>(base, (uint32_t)di.max_smem_optin, p);
+  }
   FDK_CHECK_ARG(smem != 0, FDK_ERR_CUDA, "no shared-memory plan fits %d bytes", di.max_smem_optin);
   auto kernel = gemm_lut_tc_kernel<BITS, FP16, SILU>;
   static std::atomic<bool> allowed[64] = {};
