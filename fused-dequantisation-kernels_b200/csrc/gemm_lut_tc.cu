@@ -39,6 +39,7 @@
 #include <cstring>
 
 #include "fdk_common.cuh"
+#include "gemm_cut.cuh"
 #include "lut_table.cuh"
 
 namespace fdk {
@@ -81,7 +82,7 @@ struct TcParams {
   int k_blocks, k_slabs;  // k / 64; slabs per 64-row tile
   int stages_log2, code_slots;
   int split;              // ranges may cut tiles
-  int base, rem;          // CTA `rank` owns `base + (rank < rem)` consecutive units (whole tiles where they are not cut)
+  TcCut cut;              // the CTAs' ranges of units (of whole tiles where they are not cut)
   float* partial;         // [rank][n_tile][128] fp32 sums of a CTA that does not own its first tile
   int* flags;             // [rank][column sixteenth][row quarter] the launch that published
   unsigned long long* launches;  // launches on this workspace with cut tiles
@@ -279,7 +280,7 @@ __device__ __forceinline__ int sub_tile_of(int quarter, int t) {
 
 // Unit range of CTA `rank`: units are (tile, slab) pairs, a tile's slabs consecutive.
 __device__ __forceinline__ int range_begin(const TcParams& p, int rank) {
-  const int begin = rank * p.base + min(rank, p.rem);
+  const int begin = tc_cut_begin(p.cut, rank);
   return p.split ? begin : p.k_slabs * begin;
 }
 
@@ -914,8 +915,7 @@ int gemm_rows(const void* x, const void* tiled, const void* lut, const void* lut
   }
   p.split = room >= (size_t)grid;
   if (!p.split && tiles < grid) grid = (int)tiles;
-  p.base = (int)((p.split ? units : tiles) / grid);
-  p.rem = (int)((p.split ? units : tiles) % grid);
+  p.cut = make_tc_cut((int)(p.split ? units : tiles), grid);
   CUtensorMap map;
   const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)m};
   const cuuint64_t strides[1] = {(cuuint64_t)k * 2};
