@@ -104,9 +104,10 @@ class QuantisedLinear(nn.Module):
         return self._lut_host
 
     def forward(self, x: Tensor) -> Tensor:
-        out = native.eager_linear(self.__dict__, x)
-        if out is not None:
-            return out
+        if self.kernel != "torch.compile":  # (a graph tracer cannot look into the native call)
+            out = native.eager_linear(self.__dict__, x)
+            if out is not None:
+                return out
         if x.ndim > 2:
             return self.forward(x.flatten(end_dim=-2)).unflatten(0, x.shape[:-1])
         if self.kernel == "torch.compile":

@@ -104,3 +104,13 @@ def test_what_is_left_to_the_python_code():
                  (w, 3, 64, lut), (w[:0], 4, 64, lut), (w, 4, 64, lut.half()), (w, 4, 64, lut.clone().requires_grad_())):
         assert quantise(*args, None) is None
     assert native.device_status() == 0
+
+
+@pytest.mark.parametrize("shape", [(5, 128), (2, 3, 128)])
+def test_the_torch_selector_stays_traceable(shape):
+    """A graph tracer cannot look into a native function, and layers of the plain-torch selector have no use for it."""
+    native.lib()  # binds the native calls
+    layer = models.QuantisedLinear.create(torch.randn(64, 128).bfloat16(), models.QuantisationConfig(4, 64, kernel="torch.compile"))
+    x = torch.randn(shape).bfloat16()
+    torch._dynamo.reset()
+    assert torch.equal(torch.compile(layer, backend="eager", fullgraph=True)(x), layer(x))
