@@ -160,8 +160,9 @@ class QuantisedLinear(nn.Module):
                 x.contiguous(), self.tiled(), self.lut, out, self.out_features, self.in_features, self.bits,
                 pdl=True, lut_bytes=self.lut_bytes(), silu_pairs=True,
             )
-        elif (
-            self.kernel != "torch.compile" and x.dtype == out.dtype == self.lut.dtype == torch.bfloat16 and out.is_contiguous()
+        elif (  # (what forward refuses is left to it)
+            self.kernel in ("triton", "marlin", "marlin-lut") and out.is_contiguous()
+            and x.dtype == out.dtype == self.lut.dtype == self.scale.dtype == torch.bfloat16
             and out.shape == (x.shape[0], self.out_features // 2)
         ):
             native.linear_lut_silu(

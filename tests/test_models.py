@@ -145,3 +145,27 @@ def test_quantisation_config_selector():
     cfgs = list(models._quantisation_configs([16, 4, 1], [64], ["triton", "marlin-lut"], "^lm_head$"))
     assert cfgs[0] is None
     assert [(c.bits, c.kernel) for c in cfgs[1:]] == [(4, "triton"), (4, "marlin-lut"), (1, "triton")]
+
+
+@pytest.mark.parametrize("change", ["scale", "kernel"])
+def test_gated_projection_refuses_what_forward_refuses(monkeypatch, change):
+    """Above 16 rows too: tensors of two types, and names that are no selector."""
+    from fdk import native
+
+    launched = []
+    for name in ("linear_lut", "linear_lut_silu", "silu_mul"):
+        monkeypatch.setattr(native, name, lambda *a, _n=name, **k: launched.append(_n))
+    monkeypatch.setattr(native, "repack", lambda *a: torch.zeros(0, dtype=torch.uint8))
+    layer = QuantisedLinear.create(torch.randn(128, 64).bfloat16(), QuantisationConfig(4, 64))
+    x, out = torch.randn(17, 64).bfloat16(), torch.empty((17, 64), dtype=torch.bfloat16)
+    layer.forward_silu_pairs(x, out)
+    assert launched == ["linear_lut_silu"]
+    if change == "scale":
+        layer.scale = nn.Parameter(layer.scale.half(), requires_grad=False)
+    else:
+        layer.kernel = "another"
+    with pytest.raises(AssertionError):
+        layer.forward(x)
+    with pytest.raises(AssertionError):
+        layer.forward_silu_pairs(x, out)
+    assert launched == ["linear_lut_silu"]
