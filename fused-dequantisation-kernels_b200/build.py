@@ -4,12 +4,12 @@
 
 nvcc cross-compiles without a GPU.  Objects go to csrc/build/, the shared
 library to fdk/libfdk_b200.so, the host side of eager calls (a Python extension in C++, without device
-code) to fdk/_eager.*.so; all are rebuilt only when a source is newer.
+code; left out where torch or a host compiler is missing) to fdk/_eager.*.so; all are rebuilt only when a source
+is newer, the extension also for another torch.
 """
 
 from __future__ import annotations
 
-import importlib.util
 import os
 import shutil
 import subprocess
@@ -45,19 +45,35 @@ def _newest_header() -> float:
     return max(h.stat().st_mtime for h in headers)
 
 
-def _build_eager(force: bool, verbose: bool) -> None:
-    source, header = CSRC / "eager_calls.cpp", INCLUDE / "fdk_b200.h"
-    if not force and EAGER.exists() and EAGER.stat().st_mtime >= max(source.stat().st_mtime, header.stat().st_mtime):
-        return
-    torch = Path(importlib.util.find_spec("torch").origin).parent
-    cuda = Path(_nvcc()).resolve().parents[1]
-    include = [torch / "include", torch / "include/torch/csrc/api/include", cuda / "include", Path(sysconfig.get_paths()["include"])]
-    cmd = [shutil.which("g++") or "c++", "-O2", "-std=c++17", "-fPIC", "-shared", "-D_GLIBCXX_USE_CXX11_ABI=1",
-           *(f"-I{i}" for i in include), str(source), "-o", str(EAGER), f"-L{torch / 'lib'}",
-           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python"]
-    if verbose:
-        print(" ".join(cmd), file=sys.stderr)
-    subprocess.run(cmd, check=True)
+def _build_eager(force: bool, verbose: bool) -> bool:
+    """Whether the extension is there.  The library does without torch, Python's headers and a host compiler, and the
+    package without the extension (its eager calls then take longer), so what is missing here is said and no more.
+    Torch's inline code is compiled in: another torch, or another command, makes another extension."""
+    source, header, stamp = CSRC / "eager_calls.cpp", INCLUDE / "fdk_b200.h", OBJ / "eager.stamp"
+    try:
+        import torch
+
+        root = Path(torch.__file__).parent
+        cuda = Path(_nvcc()).resolve().parents[1]
+        include = [root / "include", root / "include/torch/csrc/api/include", cuda / "include", Path(sysconfig.get_paths()["include"])]
+        cmd = [shutil.which("g++") or "c++", "-O2", "-std=c++17", "-fPIC", "-shared",
+               f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", f'-DFDK_TORCH_VERSION="{torch.__version__}"',
+               *(f"-I{i}" for i in include), str(source), "-o", str(EAGER), f"-L{root / 'lib'}",
+               "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python"]
+        made_by = "\n".join(cmd)
+        if (not force and EAGER.exists() and EAGER.stat().st_mtime >= max(source.stat().st_mtime, header.stat().st_mtime)
+                and stamp.exists() and stamp.read_text() == made_by):
+            return True
+        EAGER.unlink(missing_ok=True)
+        if verbose:
+            print(" ".join(cmd), file=sys.stderr)
+        subprocess.run(cmd, check=True)
+        stamp.write_text(made_by)
+        return True
+    except (ImportError, OSError, subprocess.CalledProcessError) as e:
+        EAGER.unlink(missing_ok=True)
+        print(f"{EAGER.name} not built ({type(e).__name__}: {e}): eager calls go through Python", file=sys.stderr)
+        return False
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:

@@ -265,5 +265,8 @@ PyMODINIT_FUNC PyInit__eager() {
       {&s_lut_key, "_lut_host_key"}, {&s_in, "in_features"}, {&s_out, "out_features"}};
   for (const auto& name : names)
     if ((*name.to = PyUnicode_InternFromString(name.text)) == nullptr) return nullptr;
-  return PyModule_Create(&module);
+  PyObject* const m = PyModule_Create(&module);
+  // torch's inline code is compiled in, so native.py binds this only beside the same torch
+  if (m != nullptr && PyModule_AddStringConstant(m, "torch_version", FDK_TORCH_VERSION) != 0) return nullptr;
+  return m;
 }

@@ -189,6 +189,8 @@ def _bind_eager(handle: ctypes.CDLL) -> None:
         from . import _eager
     except ImportError:  # not built for this interpreter: the calls take longer
         return
+    if getattr(_eager, "torch_version", None) != str(torch.__version__):  # its view of tensors is another torch's
+        return
     names = ("fdk_linear_lut", "fdk_quantise", "fdk_repack", "fdk_tiled_size")
     if all(hasattr(handle, name) for name in names):
         _eager.bind(*(ctypes.cast(getattr(handle, name), ctypes.c_void_p).value for name in names), _workspaces)
