@@ -306,12 +306,19 @@ struct Cursor {
   }
 };
 
-// SILU: out[m, n / 2] = silu(gate) * up of a weight whose rows alternate 32 gate rows and their 32 up rows, with the
-// roundings of the plain product followed by silu_mul_kernel.
-template <int BITS, bool FP16, bool SILU>
+// kTcSilu: out[m, n / 2] = silu(gate) * up of a weight whose rows alternate 32 gate rows and their 32 up rows, with the
+// roundings of the plain product followed by silu_mul_kernel.  kTcNarrow: the plain product with batch tiles of at most
+// 32 columns, whose owners fetch shares eight columns at a time: an instantiation of its own, because in the others that
+// code made the compiler spill (80 registers) and large products up to 2 % slower (1000 rows of 22528 x 3072 111.4 us, 109.1
+// without; 300 rows 39.9, 38.7).
+enum TcForm { kTcPlain, kTcSilu, kTcNarrow };
+constexpr int kTcNarrowColumns = 32;
+
+template <int BITS, bool FP16, TcForm FORM>
 __global__ void __launch_bounds__(kTcThreads, 1)
     gemm_lut_tc_kernel(const __grid_constant__ TcParams p, const __grid_constant__ InlineLut<BITS> inl,
                        const __grid_constant__ CUtensorMap x_map) {
+  constexpr bool SILU = FORM == kTcSilu;
   using L = Layout<BITS>;
   constexpr bool WIDE = kTcWideTable<BITS>;
   using T = Table<BITS, WIDE>;
@@ -409,17 +416,19 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   auto blocks_of = [&](int ks) { return KSB == 1 ? 1 : min(KSB, p.k_blocks - ks * KSB); };
 
   // ---- epilogue of one tile segment [begin, end) of slabs, by `parts` warps per 32-row quarter ----
-  auto epilogue = [&](int tile, int begin, int end, uint32_t acc, int part, int parts, int launch) {
+  auto epilogue = [&](int tile, int begin, int end, uint32_t acc, int part, auto parts_c, int launch) {
+    constexpr int parts = decltype(parts_c)::value;
     const int nt = tile / p.m_tiles, mt = tile - nt * p.m_tiles;
     const int quarter = warp & 3;
-    const int row = nt * kTcTileRows + 64 * (quarter >> 1) + 16 * sub_tile_of<SILU>(quarter, lane & 3) + 8 * (lane & 1) + (lane >> 2);
+    const int row = nt * kTcTileRows + (SILU ? 64 * (quarter >> 1) + 16 * sub_tile_of<SILU>(quarter, lane & 3) + 8 * (lane & 1) + (lane >> 2)
+                                             : 32 * quarter + 8 * (lane & 3) + (lane >> 2));
     const size_t slot = (size_t)p.n_tile * kTcTileRows;
     const uint32_t taddr = acc + ((uint32_t)(quarter * 32) << 16);
     const int tile_end = (tile + 1) * p.k_slabs;
     int last_rank = rank;  // ranks rank + 1 .. last_rank hold the rest of the tile
     if (begin == 0 && end < p.k_slabs)
       while (range_begin(p, last_rank + 1) < tile_end) ++last_rank;
-    // flag of 16 columns of 32 rows: one warp publishes them, one consumes them
+    // flag of 16 columns of 32 rows: one warp publishes them
     auto flag = [&](int of_rank, int c0) { return p.flags + of_rank * kTcFlagsPerRank + (c0 >> 4) * 4 + quarter; };
     auto await_shares = [&](int c0) {
       for (int o = rank + 1 + lane; o <= last_rank; o += 32) {  // a lane per share
@@ -442,9 +451,11 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     };
     // Several shares of a tile of few columns: eight columns at a time, so that every warp has some and the loads of four
     // shares are in flight (32 rows: 5120 x 3072 8.97 us -> 8.58, 256 x 20480 11.2 -> 9.7; with one share, or with so many
-    // columns that the warps go round twice, 16 at a time are better: 48 rows of 11264 x 3072 11.8 against 12.6).
-    if (!SILU && last_rank > rank + 1 && p.n_tile <= 8 * parts) {
-      for (int c0 = 8 * part; c0 < p.n_tile; c0 += 8 * parts) {
+    // columns that the warps go round twice, 16 at a time are better: 48 rows of 11264 x 3072 11.8 against 12.6).  Two
+    // warps then wait for one flag.
+    if (FORM == kTcNarrow && parts > 1 && last_rank > rank + 1) {
+      static_assert(parts == 1 || kTcNarrowColumns <= 8 * parts, "eight columns a warp");
+      if (const int c0 = 8 * part; c0 < p.n_tile) {
         uint32_t acc8[8];
         tmem_load8(taddr + (uint32_t)c0, acc8);
         float v[8];
@@ -505,8 +516,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             }
           }
         }
-        const int b0 = mt * p.n_tile + c0;
         if constexpr (SILU) {
+          const int b0 = mt * p.n_tile + c0;
           // a gate lane takes the even columns and the up lane two lanes on the odd ones; each sends the other its factor
           auto rnd = [](float x) { return to_float<FP16>(from_float<FP16>(x)); };
           const bool is_up = (lane & 2) != 0;
@@ -532,6 +543,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
               if (b0 + 2 * j + is_up < p.m) dst[(size_t)(2 * j) * width] = from_float<FP16>(rnd(act[j]) * up[j]);
           }
         } else if (row < p.n) {
+          const int b0 = mt * p.n_tile + c0;
           uint16_t* dst = p.out + (size_t)b0 * p.n + row;
 #pragma unroll
           for (int j = 0; j < 16; ++j)
@@ -554,8 +566,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   auto last_epilogue = [&](int part) {
     if (!mbar_wait(acc_last, 0)) timed_out = true;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    epilogue(last_tile, last_begin, last_end, acc_base + (segments - 1) % kTcAccumulators * p.n_tile, part, kSets + 1,
-             (int)ring32(launch_slot));
+    epilogue(last_tile, last_begin, last_end, acc_base + (segments - 1) % kTcAccumulators * p.n_tile, part,
+             std::integral_constant<int, kSets + 1>{}, (int)ring32(launch_slot));
   };
 
   if (segments == 0) {
@@ -648,7 +660,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       const int a = seg % kTcAccumulators;
       if (!mbar_wait(acc_full + 8 * a, (seg / kTcAccumulators) & 1)) timed_out = true;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      epilogue(tile, begin, p.k_slabs, acc_base + a * p.n_tile, 0, 1, launch);
+      epilogue(tile, begin, p.k_slabs, acc_base + a * p.n_tile, 0, std::integral_constant<int, 1>{}, launch);
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(acc_empty + 8 * a);
@@ -832,7 +844,7 @@ size_t plan_tc_smem(uint32_t base, uint32_t limit, TcParams& p) {
   return p.code_slots >= 4 ? used - base : 0;
 }
 
-template <int BITS, bool FP16, bool SILU>
+template <int BITS, bool FP16, TcForm FORM>
 int launch_tc(TcParams p, const void* lut_host, const CUtensorMap& map, int grid, bool pdl, cudaStream_t stream) {
   InlineLut<BITS> inl;
   if (lut_host != nullptr) {
@@ -855,7 +867,7 @@ int launch_tc(TcParams p, const void* lut_host, const CUtensorMap& map, int grid
     smem = plan_tc_smem<BITS>(base, (uint32_t)di.max_smem_optin, p);
   }
   FDK_CHECK_ARG(smem != 0, FDK_ERR_CUDA, "no shared-memory plan fits %d bytes", di.max_smem_optin);
-  auto kernel = gemm_lut_tc_kernel<BITS, FP16, SILU>;
+  auto kernel = gemm_lut_tc_kernel<BITS, FP16, FORM>;
   static std::atomic<bool> allowed[64] = {};
   if (int st = allow_all_smem(kernel, allowed, di)) return st;
   cudaLaunchConfig_t cfg = {};
@@ -927,9 +939,12 @@ int gemm_rows(const void* x, const void* tiled, const void* lut, const void* lut
   FDK_CHECK_ARG(r == CUDA_SUCCESS, FDK_ERR_CUDA, "cuTensorMapEncodeTiled failed with %d", (int)r);
   auto launch = [&](auto bits_c) {
     constexpr int BITS = decltype(bits_c)::value;
-    if (silu) return launch_tc<BITS, false, true>(p, lut_host, map, grid, pdl, stream);
-    return fp16 ? launch_tc<BITS, true, false>(p, lut_host, map, grid, pdl, stream)
-                : launch_tc<BITS, false, false>(p, lut_host, map, grid, pdl, stream);
+    if (silu) return launch_tc<BITS, false, kTcSilu>(p, lut_host, map, grid, pdl, stream);
+    if (p.n_tile <= kTcNarrowColumns)
+      return fp16 ? launch_tc<BITS, true, kTcNarrow>(p, lut_host, map, grid, pdl, stream)
+                  : launch_tc<BITS, false, kTcNarrow>(p, lut_host, map, grid, pdl, stream);
+    return fp16 ? launch_tc<BITS, true, kTcPlain>(p, lut_host, map, grid, pdl, stream)
+                : launch_tc<BITS, false, kTcPlain>(p, lut_host, map, grid, pdl, stream);
   };
   switch (bits) {
     case 1: return launch(std::integral_constant<int, 1>{});

@@ -52,6 +52,24 @@ def test_many_ranges_and_shapes_share_a_workspace():
     assert native.device_status() == 0
 
 
+@pytest.mark.parametrize("bits", [1, 2, 3, 4, 8])
+@pytest.mark.parametrize("m,n,k", [(17, 64, 64), (17, 100, 64 * 90), (32, 256, 64 * 320), (33, 256, 64 * 320), (32, 64 * 81, 64 * 48)])
+def test_narrow_tiles(m, n, k, bits):
+    """Tiles of up to 32 batch rows have a form of the kernel to themselves: one share, several, many, and the first size beyond."""
+    check(m, n, k, bits)
+
+
+@pytest.mark.parametrize("bits", [1, 2, 3, 4, 8])
+@pytest.mark.parametrize("m,n,k", [(17, 64, 64), (17, 100, 64 * 90), (32, 256, 64 * 320), (33, 256, 64 * 320), (32, 64 * 81, 64 * 48)])
+def test_narrow_tiles(m, n, k, bits):
+    """Tiles of up to 32 batch rows have a form of the kernel to themselves: one share, several, many, and the first size beyond."""
+    dtype = torch.float16 if m == 17 else torch.bfloat16
+    layer, x, want = problem(m, n, k, bits, dtype)
+    y = layer(x)
+    check(y, want, dtype)
+    assert torch.equal(y, layer(x)) and native.device_status() == 0
+
+
 @pytest.mark.parametrize("m,n,k", [(40, 300, 640), (300, 128, 192)])
 def test_without_room_for_partial_sums(m, n, k):
     """The scratch built into the library holds none: tiles are not cut."""

@@ -26,3 +26,9 @@ def test_code_slots_are_handed_back_behind_a_proxy_fence():
     """Plain reads and the bulk copy that refills the slot go through different proxies."""
     release = between("auto release = [&] {", "mbar_arrive(held)")
     assert release.index("fence.proxy.async.shared::cta") < release.index("__syncwarp();")
+
+
+def test_only_narrow_tiles_carry_the_eight_column_form():
+    """Compiled into the other forms it cost them registers that they spilled, and large products 2 % of their time."""
+    assert SOURCE.count("tmem_load8(") == 2  # its definition, and the one use
+    assert "if (FORM == kTcNarrow && parts > 1" in between("Several shares of a tile", "tmem_load8(taddr")
