@@ -210,10 +210,20 @@ __global__ void __launch_bounds__(kQuantThreads<TABLE>, TABLE ? 1 : 4)
         nearest = min_u16_pair(nearest, add_u16_pair(low, ((0x10000u - (Q::kTie - 8u)) & 0xFFFFu) * 0x10001u));
         least = fminf(least, fminf(fabsf(q0), fabsf(q1)));
       }
-      if ((nearest & 0xFFFFu) <= 16u || (nearest >> 16) <= 16u || least < Q::kSmall || !exact_r) {
+      const bool near = (nearest & 0xFFFFu) <= 16u || (nearest >> 16) <= 16u;
+      if (near || least < Q::kSmall || !exact_r) {
+        // Zeros are exact (pruned or padded weights: at 11264 x 3072, a tenth of them zero, 39 us at 2 bits and 43 at 4 where every
+        // octet with one divided, 31 and 37 now): the smallest magnitude beside them counts, whose pattern
+        // less one is the least when those of zeros wrap to the top.
+        uint32_t rest = 0xFFFFFFFFu;
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-          x[i] = (uint32_t)Q::exact(pair_lo<FP16>(words[i]), s, r, exact_r) | ((uint32_t)Q::exact(pair_hi<FP16>(words[i]), s, r, exact_r) << 16);
+        for (int i = 0; i < 4; ++i) rest = min_u16_pair(rest, add_u16_pair(words[i] & 0x7FFF7FFFu, 0xFFFFFFFFu));
+        const uint32_t smallest = min(rest & 0xFFFFu, rest >> 16);
+        if (near || !exact_r || (smallest != 0xFFFFu && pair_lo<FP16>(smallest + 1u) * r < Q::kSmall)) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            x[i] = (uint32_t)Q::exact(pair_lo<FP16>(words[i]), s, r, exact_r) | ((uint32_t)Q::exact(pair_hi<FP16>(words[i]), s, r, exact_r) << 16);
+        }
       }
       uint32_t packed[2] = {0u, 0u};
 #pragma unroll

@@ -71,6 +71,26 @@ def test_every_quotient_class(dtype):
     assert torch.equal(got.scale.nan_to_num(), want.scale.nan_to_num())
 
 
+@pytest.mark.parametrize("bits", [1, 2, 3, 4, 8])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_zeros_beside_small_weights(bits, dtype):
+    """Zeros need no division, the smallest values beside them do: every share of zeros in octets whose other weights make
+    quotients of all sizes, subnormal ones and such as vanish among them; codebooks with a midpoint at zero and beside it."""
+    gen = torch.Generator(device="cuda").manual_seed(bits)
+    n, k = 520, 1024
+    size = 2.0 ** torch.randint(-140 if dtype == torch.bfloat16 else -24, 1, (n, k), generator=gen, device="cuda").float()
+    w = (torch.randn((n, k), generator=gen, device="cuda") * size).to(dtype)
+    share = torch.linspace(0, 1, n, device="cuda")[:, None]
+    w = torch.where(torch.rand((n, k), generator=gen, device="cuda") < share, torch.zeros_like(w), w)
+    w[::2, ::3] *= -1  # negative zeros among them
+    tiny = torch.linspace(-1, 1, 2**bits, device="cuda") * (2.0**-130 if dtype == torch.bfloat16 else 2.0**-22)
+    for lut in (torch.linspace(-1, 1, 2**bits, device="cuda").to(dtype), tiny.to(dtype)):
+        config = models.QuantisationConfig(bits, 64)
+        got, want = models.QuantisedLinear.create(w, config, lut=lut), by_torch(w, config, lut)
+        assert torch.equal(got.weight_data, want.weight_data)
+        assert torch.equal(got.scale.view(torch.int16), want.scale.view(torch.int16))
+
+
 def test_other_weights_keep_the_general_path():
     w = torch.randn((64, 128), device="cuda").bfloat16()
     lut = torch.linspace(-1, 1, 16, device="cuda", dtype=torch.bfloat16)
