@@ -154,11 +154,15 @@ __device__ __forceinline__ int div_k(const LinearParams& p, int n) {  // see lin
 }
 __device__ __forceinline__ int cta_begin(const LinearParams& p, int c) { return c * p.base + min(c, p.rem); }
 
-// FUSED: with the outputs and the norm factors of the decode fusions and of the tensor-parallel push; the plain kernel
-// carries none of their code (0.3 us of 6 to 12).
-template <int BITS, int NB, bool FP16, bool FUSED>
+// kFused: with the norm factors of the decode fusions and the rotary and tensor-parallel outputs.  kResid: with the norm
+// factors and the residual output.  The plain kernel carries none of their code (0.3 us of 6 to 12), and they not
+// each other's: in one, the registers of the residual output cost the others up to 15 % (3 bits, one n-tile, 28672 x
+// 4096 with SiLU 29.8 us, 25.2 apart).
+enum Form { kLean, kFused, kResid };
+template <int BITS, int NB, bool FP16, Form FORM>
 __global__ void __launch_bounds__(32 * kWarps<NB>, 1)
     skinny_lut_kernel(const __grid_constant__ LinearParams p, const __grid_constant__ InlineLut<BITS> inl) {
+  constexpr bool FUSED = FORM != kLean;
   using L = Layout<BITS>;
   constexpr bool WIDE = BITS != 3;
   using Tab = Table<BITS, WIDE>;
@@ -172,7 +176,7 @@ __global__ void __launch_bounds__(32 * kWarps<NB>, 1)
   const int g = lane >> 2, t = lane & 3;
   const int tile = warp & (kTiles - 1), phase = warp / kTiles;
   const uint32_t table_addr = raw + p.table_off;
-  const Epilogue epi = FUSED ? (Epilogue)p.epilogue : p.silu ? kSilu : kStore;
+  const Epilogue epi = FORM == kResid ? kResidual : FORM == kFused ? (Epilogue)p.epilogue : p.silu ? kSilu : kStore;
   const uint32_t ring = raw + p.xres_off + phase * (kRing * kSlot);
 
   // waits go to CTAs of lower block index, which the GPU starts first
@@ -250,7 +254,7 @@ __global__ void __launch_bounds__(32 * kWarps<NB>, 1)
   for (int d = 0; d < kRing - 1; ++d) copy_x();
   const int uses_first = ld_relaxed_s32(p.counters + first), uses_last = ld_relaxed_s32(p.counters + last);
   uint32_t push_seq = 0;
-  if (FUSED && epi == kPush) push_seq = (uint32_t)ld_relaxed_s32(reinterpret_cast<const int*>(p.seq));  // reduces completed so far
+  if (FORM == kFused && epi == kPush) push_seq = (uint32_t)ld_relaxed_s32(reinterpret_cast<const int*>(p.seq));  // reduces completed so far
   if constexpr (FUSED) {
     // what only the epilogues read: the deferred RMSNorm's factors (the row's sums of squares added in a fixed order; 1
     // without it), the position and its cos/sin table
@@ -271,7 +275,7 @@ __global__ void __launch_bounds__(32 * kWarps<NB>, 1)
       }
       if (lane == 0) inv[b] = p.scale_ss != nullptr && b < p.m ? rsqrtf(sum / (float)p.k + p.scale_eps) : 1.f;
     }
-    if (epi == kRotary && warp == kWarps<NB> - 1) {
+    if (FORM == kFused && epi == kRotary && warp == kWarps<NB> - 1) {
       uint32_t* const table = reinterpret_cast<uint32_t*>(smem_raw + kHeadRope);
       table[lane] = __ldcg(p.rope_table + lane);
       table[lane + 32] = __ldcg(p.rope_table + lane + 32);
@@ -296,13 +300,56 @@ __global__ void __launch_bounds__(32 * kWarps<NB>, 1)
     const uint32_t slot = (uint32_t)((of_warp * kUnits + unit) * 2 + half);
     return raw + p.slots_off + slot * 512 + lane * 16;
   };
+  // What the residual output reads for a unit, asked for together and ahead of the sums: h is read and written, so loads
+  // left beside the stores wait for them one by one (eight trips to L2 at two rows and more: 3 rows of 3072^2, 4 bits
+  // 8.5 us, 6.0 this way).
+  struct Residual {
+    uint16_t h[FORM == kResid ? 2 : 1][4], w[FORM == kResid ? 2 : 1][2];
+  };
+  auto fetch_residual = [&](int rt, int q, int nb, Residual& r) {
+    if constexpr (FORM == kResid) {
+      const int row0 = rt * kTileRows + 16 * q + g;
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int b = 8 * nb + 2 * t + (i & 1), row = row0 + 32 * h + 8 * (i >> 1);
+          r.h[h][i] = b < p.m && row < p.n ? __ldcg(p.resid_h + (size_t)b * p.n + row) : (uint16_t)0;
+          if ((i & 1) == 0) r.w[h][i >> 1] = p.resid_w != nullptr && row < p.n ? __ldg(p.resid_w + row) : (uint16_t)0;
+        }
+    }
+  };
   // The end of the sub-tiles q and q + 2 of row tile rt, batch rows 8 nb .. 8 nb + 7: sum[h][i] is row
   // 16 q + 32 h + g + 8 (i / 2) of the tile, batch row 8 nb + 2 t + i % 2.
-  auto finish = [&](int rt, int q, int nb, const float (&sum)[2][4]) {
+  auto finish = [&](int rt, int q, int nb, const float (&sum)[2][4], const Residual& res) {
     auto rnd = [](float v) { return to_float<FP16>(from_float<FP16>(v)); };
     const int row0 = rt * kTileRows + 16 * q + g;  // row of sum[0][0]
     const bool live = rt < row_tiles;
-    if (FUSED && epi == kPush) {
+    if constexpr (FORM == kResid) {
+      // y rounded as if stored, added to the residual stream; sums of squares over the lanes of a batch row
+      float sq[2] = {0.f, 0.f};
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int b = 8 * nb + 2 * t + (i & 1), row = row0 + 32 * h + 8 * (i >> 1);
+          if (live && b < p.m && row < p.n) {
+            const size_t at = (size_t)b * p.n + row;
+            const uint16_t hnew = from_float<FP16>(to_float<FP16>(res.h[h][i]) + rnd(sum[h][i]));
+            p.resid_h[at] = hnew;
+            const float hf = to_float<FP16>(hnew);
+            sq[i & 1] = fmaf(hf, hf, sq[i & 1]);
+            if (p.resid_w != nullptr)  // the next RMSNorm's weight folded in: x of the next projection
+              p.resid_x[at] = from_float<FP16>(hf * to_float<FP16>(res.w[h][i >> 1]));
+          }
+        }
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) sq[j] += __shfl_xor_sync(0xffffffffu, sq[j], o);
+        if (g == 0) reinterpret_cast<float*>(smem_raw + kHeadSq)[(tile * 2 + q) * 8 * NB + 8 * nb + 2 * t + j] = sq[j];
+      }
+    } else if (FORM == kFused && epi == kPush) {
       // four consecutive rows (four lanes) as two words {two outputs, tag}, into every rank's exchange buffer
       const uint32_t ptag = push_seq + 1u;
       const size_t base = (size_t)((push_seq & 1u) * p.tp + p.rank) * p.stage_slot;
@@ -323,33 +370,9 @@ __global__ void __launch_bounds__(32 * kWarps<NB>, 1)
                            : "memory");
           }
         }
-    } else if (FUSED && epi == kResidual) {
-      // y rounded as if stored, added to the residual stream; sums of squares over the lanes of a batch row
-      float sq[2] = {0.f, 0.f};
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int b = 8 * nb + 2 * t + (i & 1), row = row0 + 32 * h + 8 * (i >> 1);
-          if (live && b < p.m && row < p.n) {
-            const size_t at = (size_t)b * p.n + row;
-            const uint16_t hnew = from_float<FP16>(to_float<FP16>(__ldcg(p.resid_h + at)) + rnd(sum[h][i]));
-            p.resid_h[at] = hnew;
-            const float hf = to_float<FP16>(hnew);
-            sq[i & 1] = fmaf(hf, hf, sq[i & 1]);
-            if (p.resid_w != nullptr)  // the next RMSNorm's weight folded in: x of the next projection
-              p.resid_x[at] = from_float<FP16>(hf * to_float<FP16>(__ldg(p.resid_w + row)));
-          }
-        }
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-#pragma unroll
-        for (int o = 4; o < 32; o <<= 1) sq[j] += __shfl_xor_sync(0xffffffffu, sq[j], o);
-        if (g == 0) reinterpret_cast<float*>(smem_raw + kHeadSq)[(tile * 2 + q) * 8 * NB + 8 * nb + 2 * t + j] = sq[j];
-      }
     } else if (live) {
-      const long long pos = FUSED ? *reinterpret_cast<const long long*>(smem_raw + kHeadPos) : 0;
-      const bool in_cache = FUSED && epi == kRotary && pos >= 0 && pos < p.max_len;
+      const long long pos = FORM == kFused ? *reinterpret_cast<const long long*>(smem_raw + kHeadPos) : 0;
+      const bool in_cache = FORM == kFused && epi == kRotary && pos >= 0 && pos < p.max_len;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int b = 8 * nb + 2 * t + (i & 1), lrow = 16 * q + g + 8 * (i >> 1);  // of 32: the partner is 32 rows on
@@ -358,7 +381,7 @@ __global__ void __launch_bounds__(32 * kWarps<NB>, 1)
           uint16_t* const dst = p.out + (size_t)b * p.n + rt * kTileRows + lrow;
           if (rt * kTileRows + lrow < p.n) dst[0] = from_float<FP16>(sum[0][i]);
           if (rt * kTileRows + lrow + 32 < p.n) dst[32] = from_float<FP16>(sum[1][i]);
-        } else if (!FUSED || epi == kSilu) {  // rows come as 32 gate + 32 up
+        } else if (FORM == kLean || epi == kSilu) {  // rows come as 32 gate + 32 up
           const float gate = rnd(sum[0][i]), up = rnd(sum[1][i]);
           p.out[(size_t)b * (p.n / 2) + rt * (kTileRows / 2) + lrow] = from_float<FP16>(rnd(gate / (1.f + __expf(-gate))) * up);
         } else {  // rotary: tile rt is half th of head rt / 2; dimensions 32 th + lrow and 64 further on
@@ -384,12 +407,14 @@ __global__ void __launch_bounds__(32 * kWarps<NB>, 1)
       }
     }
   };
-  // Finishes groups cur .. target - 1: every warp deposits its sums, the owner of a unit adds the four phases
+  // Finishes groups cur .. target - 1: every warp deposits its sums, the owner of a unit adds the phases
   // in order, and writes the outputs, publishes the sums (a group that starts in another CTA), or adds the
   // sums of the CTAs that hold the rest of the group.
   auto flush_until = [&](int target) {
 #pragma unroll 1
     while (cur < target) {
+      const int lo = cur * p.k_slabs, hi = lo + p.k_slabs;
+      const bool owner = c0 <= lo, full = owner && c1 >= hi;
 #pragma unroll
       for (int q = 0; q < 2; ++q)
 #pragma unroll
@@ -402,9 +427,9 @@ __global__ void __launch_bounds__(32 * kWarps<NB>, 1)
                          : "memory");
             v[0] = v[1] = v[2] = v[3] = 0.f;
           }
+      Residual res;
+      if (FORM == kResid && owner && phase < kUnits) fetch_residual(cur + tile * groups, phase / NB, phase % NB, res);
       __syncthreads();
-      const int lo = cur * p.k_slabs, hi = lo + p.k_slabs;
-      const bool owner = c0 <= lo, full = owner && c1 >= hi;
       const int uses = cur == first ? uses_first : uses_last;  // only those two can be split
       const uint32_t tag = ((uint32_t)(uses + 1) << 12) | (uint32_t)cur;
       if (phase < kUnits) {
@@ -472,12 +497,12 @@ __global__ void __launch_bounds__(32 * kWarps<NB>, 1)
 #pragma unroll
               for (int i = 0; i < 4; ++i) sum[h][i] *= inv[i & 1];
           }
-          finish(cur + tile * groups, q, nb, sum);
+          finish(cur + tile * groups, q, nb, sum, res);
         }
       }
       __syncthreads();  // the deposits have been read; everybody is done with the foreign sums
       if (!full && owner && threadIdx.x == 0) p.counters[cur] = (uses + 1) & 0x7FFFF;
-      if (FUSED && epi == kResidual && owner && threadIdx.x < kTiles * 8 * NB) {
+      if (FORM == kResid && owner && threadIdx.x < kTiles * 8 * NB) {
         const int of_tile = threadIdx.x / (8 * NB), b = threadIdx.x % (8 * NB), rt = cur + of_tile * groups;
         const float* const sq = reinterpret_cast<const float*>(smem_raw + kHeadSq) + of_tile * 2 * 8 * NB + b;
         if (b < p.m && rt < row_tiles) p.resid_ss[(size_t)b * row_tiles + rt] = sq[0] + sq[8 * NB];
@@ -580,7 +605,7 @@ __global__ void __launch_bounds__(32 * kWarps<NB>, 1)
 
 // ---- host side ----------------------------------------------------------------------------------------------
 
-template <int BITS, int NB, bool FP16, bool FUSED>
+template <int BITS, int NB, bool FP16, Form FORM>
 int launch_kernel(LinearParams p, const InlineLut<BITS>& inl, int sm_count, unsigned flags, cudaStream_t stream) {
   constexpr int kThreads = 32 * kWarps<NB>, kPhases = kWarps<NB> / kTiles;
   uint32_t base = 0;
@@ -607,7 +632,7 @@ int launch_kernel(LinearParams p, const InlineLut<BITS>& inl, int sm_count, unsi
   if (best < grid) grid = best < 1.0 ? 1 : (int)best;
   p.base = p.total / grid;
   p.rem = p.total % grid;
-  auto kernel = skinny_lut_kernel<BITS, NB, FP16, FUSED>;
+  auto kernel = skinny_lut_kernel<BITS, NB, FP16, FORM>;
   static std::atomic<bool> allowed[64] = {};
   if (int st = allow_all_smem(kernel, allowed, di)) return st;
   cudaLaunchConfig_t cfg = {};
@@ -626,9 +651,12 @@ int launch_kernel(LinearParams p, const InlineLut<BITS>& inl, int sm_count, unsi
 
 template <int BITS, int NB, bool FP16>
 int launch(const LinearParams& p, const InlineLut<BITS>& inl, int sm_count, unsigned flags, cudaStream_t stream) {
-  const bool fused = p.tp > 0 || p.resid_h != nullptr || p.rope_pos != nullptr || p.scale_ss != nullptr;
-  return fused ? launch_kernel<BITS, NB, FP16, true>(p, inl, sm_count, flags, stream)
-               : launch_kernel<BITS, NB, FP16, false>(p, inl, sm_count, flags, stream);
+  const bool fused = p.tp > 0 || p.rope_pos != nullptr || p.scale_ss != nullptr;
+  if constexpr (!FP16) {  // (the decode fusions take bf16)
+    if (p.resid_h != nullptr) return launch_kernel<BITS, NB, FP16, kResid>(p, inl, sm_count, flags, stream);
+  }
+  return fused ? launch_kernel<BITS, NB, FP16, kFused>(p, inl, sm_count, flags, stream)
+               : launch_kernel<BITS, NB, FP16, kLean>(p, inl, sm_count, flags, stream);
 }
 
 }  // namespace
