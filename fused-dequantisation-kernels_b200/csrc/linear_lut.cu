@@ -65,11 +65,31 @@ extern "C" int fdk_workspace_status(const void* workspace, int* status_host) {
   return FDK_OK;
 }
 
-// From how many rows on the kernel for batches that share x (skinny_lut_kernel.cuh) is the faster one (up to 16 rows), us per
-// launch in a graph, linear_lut_kernel.cuh / that one: 4 bits, 2 rows, 8192^2 11.0 / 12.0, 3072^2 4.4 / 5.6; 3 rows 12.05 /
-// 12.06, 5.8 / 5.7; 2 bits, 3 rows 11.1 / 11.8, 6.4 / 5.9; 5 rows of 14336 x 4096 13.2 / 11.0; one row of 8192^2: 3 bits
-// 16.4 / 12.6, 1 bit 12.2 / 11.4, 8 bits 27.1 / 18.1.
-static int skinny_rows(int bits) { return bits == 4 ? 3 : bits == 2 ? 5 : 1; }
+// Whether the kernel for batches that share x (skinny_lut_kernel.cuh) is the faster one, up to 16 rows.  From five rows on it
+// is, at every width and size; below, its loop is the better one at 1, 3 and 8 bits and its group ends are dearer: they
+// weigh least where rows are short, or where a multiprocessor has much work beside them.  The line is
+// drawn by the plain product (a fused one then gives the same sums), with an eye on the fused ones; us per launch in a
+// graph, linear_lut_kernel.cuh / that one, plain, 37 sizes measured:
+//   three and four rows   4 bits 3072^2 5.9 / 5.6, 1024 x 8192 7.9 / 6.6, 6144 x 4096 7.4 / 7.5, 8192^2 11.6 / 12.4, 22528 x
+//                         3072 12.7 / 12.8; 2 bits 3072^2 6.5 / 5.7, 4096^2 6.7 / 6.8, 8192^2 11.2 / 12.0; 1, 3 and 8 bits the
+//                         other one throughout (4096^2 8.1 / 6.8, 8.6 / 7.6, 10.3 / 8.3)
+//   one and two rows      4 bits 8192^2 11.0 / 12.0, 3072^2 4.4 / 5.6, 2 bits 9.8 / 11.8 and 4.9 / 5.9 (never);
+//                         8 bits 3072^2 6.6 / 6.5, 1024 x 8192 7.0 / 7.7, 4096^2 9.1 / 8.2, 8192^2 25.3 / 18.7;
+//                         3 bits 3072^2 6.7 / 5.7, 4096^2 7.3 / 7.5, 3072 x 8192 8.3 / 8.8, 8192^2 17.0 / 12.6;
+//                         1 bit 3072^2 6.7 / 5.3, 4096^2 6.9 / 6.7, 6144 x 4096 7.4 / 7.7, 3072 x 11264 7.9 / 8.6, 8192^2 11.8 / 11.4
+// At 3 bits the fused forms spill at a group's end (one n-tile, 168 registers), and where rows are shorter than 3072 a
+// multiprocessor has two of them: residual output, one row, 2048^2 7.3 / 7.9, 3072^2 7.3 / 6.7.
+static bool skinny_pays(int bits, int m, int n, int k, int sm_count, bool fused) {
+  if (m >= 5) return true;
+  const long long share = (long long)n * k / sm_count;  // weights of a multiprocessor
+  if (bits == 2 || bits == 4) return m >= 3 && (k < 4096 || share < (128 << 10));
+  if (m >= 3) return true;
+  switch (bits) {
+    case 1: return k < 4096 || (k < 8192 ? share < (128 << 10) : share >= (300 << 10));
+    case 3: return (k < 4096 && !(fused && k < 3072)) || share >= (300 << 10);
+    default: return k < 4096 || share >= (64 << 10);
+  }
+}
 
 // skinny_partial: kSkinnyPartialBytes of scratch that hold nothing else, or null (a workspace of an older size).
 static int linear_lut_impl(const void* x, const void* tiled, const void* lut, const void* lut_host, void* out,
@@ -184,7 +204,7 @@ static int linear_lut_impl(const void* x, const void* tiled, const void* lut, co
     return gemm_lut_tc(x, tiled, lut, lut_host, out, m, n, k, bits, dtype == FDK_DTYPE_F16, false, workspace, workspace_bytes,
                        di.sm_count, (flags & FDK_FLAG_PDL) != 0, (cudaStream_t)stream);
   }
-  if (skinny_partial != nullptr && !norm && m >= skinny_rows(bits) && m <= 16) {
+  if (skinny_partial != nullptr && !norm && m <= 16 && skinny_pays(bits, m, n, k, di.sm_count, fu != nullptr)) {
     p.m = m;
     p.x = (const uint16_t*)x;
     p.out = (uint16_t*)out;

@@ -626,10 +626,11 @@ int launch_kernel(LinearParams p, const InlineLut<BITS>& inl, int sm_count, unsi
   p.total = groups * p.k_slabs;
   // One CTA per SM, fewer where so many would share a group that fetching their sums (about 0.2 us a CTA) costs
   // more than they save (a slab takes a warp about 0.9 us): total / (grid phases) 0.9 + grid / groups 0.2 is least at
-  // the root below (256 x 20480, 3 rows: 20.2 us with 148 CTAs).
+  // the root below (256 x 20480, 3 rows: 20.2 us with 148 CTAs).  Not fewer than groups: with as many none is shared
+  // (256^2, one row at 1 bit, two groups of one slab: 4.8 us in one CTA, 3.2 in two).
   const double best = std::sqrt((double)p.total * groups * (0.9 / 0.2) / kPhases);
   int grid = p.total < sm_count ? p.total : sm_count;
-  if (best < grid) grid = best < 1.0 ? 1 : (int)best;
+  if (best < grid) grid = best < groups ? (groups < grid ? groups : grid) : (int)best;
   p.base = p.total / grid;
   p.rem = p.total % grid;
   auto kernel = skinny_lut_kernel<BITS, NB, FP16, FORM>;
