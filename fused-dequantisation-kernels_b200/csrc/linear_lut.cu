@@ -68,8 +68,7 @@ extern "C" int fdk_workspace_status(const void* workspace, int* status_host) {
 // Whether the kernel for batches that share x (skinny_lut_kernel.cuh) is the faster one, up to 16 rows.  From five rows on it
 // is, at every width and size; below, its loop is the better one at 1, 3 and 8 bits and its group ends are dearer: they
 // weigh least where rows are short, or where a multiprocessor has much work beside them.  The line is
-// drawn by the plain product (a fused one then gives the same sums), with an eye on the fused ones; us per launch in a
-// graph, linear_lut_kernel.cuh / that one, plain, 37 sizes measured:
+// drawn by the plain product, us per launch in a graph, linear_lut_kernel.cuh / that one, 37 sizes measured:
 //   three and four rows   4 bits 3072^2 5.9 / 5.6, 1024 x 8192 7.9 / 6.6, 6144 x 4096 7.4 / 7.5, 8192^2 11.6 / 12.4, 22528 x
 //                         3072 12.7 / 12.8; 2 bits 3072^2 6.5 / 5.7, 4096^2 6.7 / 6.8, 8192^2 11.2 / 12.0; 1, 3 and 8 bits the
 //                         other one throughout (4096^2 8.1 / 6.8, 8.6 / 7.6, 10.3 / 8.3)
@@ -77,12 +76,15 @@ extern "C" int fdk_workspace_status(const void* workspace, int* status_host) {
 //                         8 bits 3072^2 6.6 / 6.5, 1024 x 8192 7.0 / 7.7, 4096^2 9.1 / 8.2, 8192^2 25.3 / 18.7;
 //                         3 bits 3072^2 6.7 / 5.7, 4096^2 7.3 / 7.5, 3072 x 8192 8.3 / 8.8, 8192^2 17.0 / 12.6;
 //                         1 bit 3072^2 6.7 / 5.3, 4096^2 6.9 / 6.7, 6144 x 4096 7.4 / 7.7, 3072 x 11264 7.9 / 8.6, 8192^2 11.8 / 11.4
-// At 3 bits the fused forms spill at a group's end (one n-tile, 168 registers), and where rows are shorter than 3072 a
-// multiprocessor has two of them: residual output, one row, 2048^2 7.3 / 7.9, 3072^2 7.3 / 6.7.
+// The fused outputs follow it but for two cases.  Three and four rows at 2 and 4 bits: the residual output gains throughout (4
+// bits, 3 rows, 8192^2 13.6 / 13.1), and a step whose projections change between kernels pays for it at every change (8
+// layers of 4B widths, 4 bits, 3 sequences 427 us with both, 414 with one; 6 of 12B widths 405, 401).  3 bits: those outputs spill at a
+// group's end (one n-tile, 168 registers), and where rows are shorter than 3072 a multiprocessor has two of them:
+// residual output, one row, 2048^2 7.3 / 7.9, 3072^2 7.3 / 6.7.
 static bool skinny_pays(int bits, int m, int n, int k, int sm_count, bool fused) {
   if (m >= 5) return true;
   const long long share = (long long)n * k / sm_count;  // weights of a multiprocessor
-  if (bits == 2 || bits == 4) return m >= 3 && (k < 4096 || share < (128 << 10));
+  if (bits == 2 || bits == 4) return m >= 3 && (fused || k < 4096 || share < (128 << 10));
   if (m >= 3) return true;
   switch (bits) {
     case 1: return k < 4096 || (k < 8192 ? share < (128 << 10) : share >= (300 << 10));
