@@ -25,7 +25,7 @@
 // the store of the tile and the MMA's reads of it out of shared memory, and its MMAs of
 // small N are faster (a block at N = 32 takes 68 cycles, 161 with A in shared memory).  Before (A in
 // shared memory, eight dequantising warps, a tile per CTA) and now, 4 bits, public call: 48 rows of
-// 11264 x 3072, four in a graph, 92.4 -> 52.0 us; 2048 rows of 28672 x 4096 792 -> 406 to 428 us, by the clock
+// 11264 x 3072, four in a graph, 92.4 -> 51.0 us; 2048 rows of 28672 x 4096 792 -> 403 to 428 us, by the clock
 // (1.12 to 1.19 PFLOP/s).  Tried and not kept: groups of four blocks per copy, barrier and stage (18.4 us at
 // 32 rows of 8192^2 against 16.7, kernel alone: a set then waits for a whole group, and the larger
 // stages leave fewer of them).

@@ -1,6 +1,10 @@
 // Fused dequantise + GEMV / skinny GEMM for sm_100a:  out[m, n] = x[m, k] . W[n, k]^T,
 // W given as tiled low-bit codes + block scales + a lookup table (fdk_layout.cuh).
 //
+// It serves up to four rows where it is the faster one (skinny_pays in linear_lut.cu), the fused RMSNorm on the
+// input, and, for callers whose workspace has an older size, all of 1 to 16 rows; the rest up to 16 is
+// skinny_lut_kernel.cuh's.
+//
 // Shape of the kernel (one persistent CTA per SM: 19 compute warps and one finisher warp for
 // batches up to 8 rows, 11 + 1 for 9 to 16 rows):
 //   * The weight stream is cut into slabs (64 rows x 64*KSB columns, 2-6 KB).  The
@@ -168,11 +172,6 @@ constexpr int kEpiStore = 0, kEpiSilu = 1, kEpiPush = 2, kEpiResid = 3, kEpiRope
 // position and the cos/sin table of the rotary epilogue.
 constexpr uint32_t kSmemInv = 32, kSmemPos = 96, kSmemRope = 128, kSmemHead = 512;
 
-// n / k_slabs for n * k_slabs < 2^32, by multiplication with k_magic = ceil(2^32 / k_slabs)
-__device__ __forceinline__ int div_k(const LinearParams& p, int n) {
-  return p.k_slabs == 1 ? n : (int)__umulhi((uint32_t)n, p.k_magic);
-}
-__device__ __forceinline__ int cta_begin(const LinearParams& p, int c) { return c * p.base + min(c, p.rem); }
 __device__ __forceinline__ int cta_of(const LinearParams& p, int item) {
   const int big = p.rem * (p.base + 1);
   return item < big ? item / (p.base + 1) : p.rem + (item - big) / p.base;
@@ -483,14 +482,6 @@ struct SlabRegs {
   uint4 sc[Layout<BITS>::KSB];
 };
 
-// Streaming load: weights are read once, so they are kept out of L1.
-__device__ __forceinline__ uint4 ldg_stream(const uint8_t* p) {
-  uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "l"(p));
-  return v;
-}
 // x: written by the previous kernel on the stream, read through L2.
 __device__ __forceinline__ uint4 ldg_l2(const void* p) {
   uint4 v;
@@ -507,13 +498,6 @@ __device__ __forceinline__ void ldg_l2_if(bool live, const void* p, uint4& lo, u
       : "+r"(lo.x), "+r"(lo.y), "+r"(lo.z), "+r"(lo.w), "+r"(hi.x), "+r"(hi.y), "+r"(hi.z), "+r"(hi.w)
       : "l"(p), "r"((uint32_t)live)
       : "memory");
-}
-
-// Asks L2 for one whole slab (a hint: no registers, no shared memory).  One bulk request instead of a
-// prefetch per line: those pass through the shared-memory pipe, which the lookups need, 17 wavefronts a slab.
-template <int BITS>
-__device__ __forceinline__ void prefetch_slab_l2(const uint8_t* slab, int lane) {
-  if (lane == 0) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(slab), "n"(Layout<BITS>::kSlabBytes));
 }
 
 template <int BITS>
@@ -592,7 +576,7 @@ __global__ void __launch_bounds__((WARPS + 1) * 32, 1)
   SlabRegs<BITS> s, s2;
   if (warp < W && it < c1) {
     load_slab<BITS>(s, wp, lane);
-    if (it + W < c1) prefetch_slab_l2<BITS>(wp + kStep, lane);
+    if (it + W < c1 && lane == 0) prefetch_slab<BITS>(wp + kStep);
   }
   {
     const bool from_params = p.lut == nullptr;
@@ -992,7 +976,7 @@ __global__ void __launch_bounds__((WARPS + 1) * 32, 1)
     if (it >= c1) return false;
     if (rt != cur_rt) flush_until(rt);
     if (it + W < c1) load_slab<BITS>(nxt, wp + kStep, lane);
-    if (it + 2 * W < c1) prefetch_slab_l2<BITS>(wp + 2 * (size_t)kStep, lane);
+    if (it + 2 * W < c1 && lane == 0) prefetch_slab<BITS>(wp + 2 * (size_t)kStep);
     compute(cur, ks);
     wp += kStep;
     it += W;

@@ -70,6 +70,28 @@ struct LinearParams {
   int epilogue;             // (skinny kernel) what is done with finished sums
 };
 
+// n / k_slabs for n * k_slabs < 2^32, by multiplication with k_magic = ceil(2^32 / k_slabs)
+__device__ __forceinline__ int div_k(const LinearParams& p, int n) {
+  return p.k_slabs == 1 ? n : (int)__umulhi((uint32_t)n, p.k_magic);
+}
+__device__ __forceinline__ int cta_begin(const LinearParams& p, int c) { return c * p.base + min(c, p.rem); }
+
+// Streaming load: weights are read once, so they are kept out of L1.
+__device__ __forceinline__ uint4 ldg_stream(const uint8_t* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p));
+  return v;
+}
+
+// Asks L2 for one whole slab (a hint: no registers, no shared memory), from one lane.  One bulk request instead of a
+// prefetch per line: those pass through the shared-memory pipe, which the lookups need, 17 wavefronts a slab.
+template <int BITS>
+__device__ __forceinline__ void prefetch_slab(const uint8_t* slab) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(slab), "n"(Layout<BITS>::kSlabBytes));
+}
+
 // Plans shared memory and launches; one explicit instantiation per code width, each in a
 // translation unit of its own so that they compile in parallel.
 template <int BITS>

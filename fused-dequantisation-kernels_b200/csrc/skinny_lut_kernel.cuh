@@ -9,7 +9,7 @@
 //     owns a contiguous range (stream-K), its phases taking slab columns in turn.
 //   * The two warps of a phase share x: each copies half of a 64-column block of it into a ring in shared memory
 //     (cp.async, three blocks ahead), so x is read from L2 once per 128 rows and its latency does not show.
-//   * With 168 to 255 registers the lookups of one sub-tile run beside the MMAs of another, and every code vector is
+//   * With 157 to 255 registers (at 3 bits and one n-tile 168, and spills) the lookups of one sub-tile run beside the MMAs of another, and every code vector is
 //     replaced by the next slab's as soon as it has been used.  8192^2, 16 rows, 4 bits, eight warps: 16.2 us at 128
 //     registers, 14.0 with all; one n-tile, 8 rows: 12.8 us with eight warps, 12.0 with twelve of 168 registers.
 //   * At the end of a group the warps deposit their sums; each (tile, pair of sub-tiles, n-tile) is added up by one
@@ -125,13 +125,6 @@ __device__ __forceinline__ void build_fragments(const uint4 (&code)[Layout<BITS>
   }
 }
 
-__device__ __forceinline__ uint4 ldg_stream(const uint8_t* p) {  // weights are read once: kept out of L1
-  uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "l"(p));
-  return v;
-}
 __device__ __forceinline__ uint4 ld_relaxed_v4(const uint4* p) {
   uint4 v;
   asm volatile("ld.relaxed.gpu.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
@@ -143,16 +136,6 @@ __device__ __forceinline__ void st_relaxed_v4(uint4* p, uint4 v) {
 
 // What is done with the finished sums of a tile (a value of the launch: it is looked at once per group).
 enum Epilogue { kStore, kSilu, kPush, kResidual, kRotary };
-
-template <int BITS>
-__device__ __forceinline__ void prefetch_slab(const uint8_t* slab) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(slab), "n"(Layout<BITS>::kSlabBytes));
-}
-
-__device__ __forceinline__ int div_k(const LinearParams& p, int n) {  // see linear_lut_kernel.cuh
-  return p.k_slabs == 1 ? n : (int)__umulhi((uint32_t)n, p.k_magic);
-}
-__device__ __forceinline__ int cta_begin(const LinearParams& p, int c) { return c * p.base + min(c, p.rem); }
 
 // kFused: with the norm factors of the decode fusions and the rotary and tensor-parallel outputs.  kResid: with the norm
 // factors and the residual output.  The plain kernel carries none of their code (0.3 us of 6 to 12), and they not

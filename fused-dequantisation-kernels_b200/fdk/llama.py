@@ -125,10 +125,10 @@ class LlamaDecoder(nn.Module):
         # the 4B shape, tokens/s split / while copying: batch 1: 754 / 740, 2: 1456 / 1426,
         # 4: 2426 / 2298
         self.deferred_norm = True
-        # largest batch whose projections carry the decode-step fusions.  Measured on the 4B shape
-        # (tokens/s fused against separate glue kernels): batch 1: 754 / 719, 2: 1456 / 1397,
-        # 4: 2426 / 2374, 8: 3780 / 3838 -- the single finisher warp goes through all batch rows,
-        # and the small glue kernels overlap their neighbours well
+        # largest batch whose projections carry the decode-step fusions.  Drawn for the GEMV kernel, whose
+        # single finisher warp goes through all batch rows; from three or five rows on another kernel
+        # without such a warp serves them, with which the fusions pay up to 16 rows (8 layers of 4B
+        # widths, 4 bits, us a step fused / separate: 5 rows 425 / 471, 8: 443 / 500, 16: 544 / 574).  Left at 4 because a larger one changes logits: the split norm rounds x elsewhere
         self.fuse_rows = 4
         # largest batch whose q|k|v projection does the rotary embedding + KV append in its epilogue
         # in the tensor-parallel step (where the norms cannot be fused)
