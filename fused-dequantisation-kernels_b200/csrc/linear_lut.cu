@@ -66,7 +66,7 @@ extern "C" int fdk_workspace_status(const void* workspace, int* status_host) {
 }
 
 // Whether the kernel for batches that share x (skinny_lut_kernel.cuh) is the faster one, up to 16 rows.  From five rows on it
-// is, at every width and size; below, its loop is the better one at 1, 3 and 8 bits and its group ends are dearer: they
+// is (or within 3 %, at 4 bits), at every width and size; below, its loop is the better one at 1, 3 and 8 bits and its group ends are dearer: they
 // weigh least where rows are short, or where a multiprocessor has much work beside them.  The line is
 // drawn by the plain product, us per launch in a graph, linear_lut_kernel.cuh / that one, 37 sizes measured:
 //   three and four rows   4 bits 3072^2 5.9 / 5.6, 1024 x 8192 7.9 / 6.6, 6144 x 4096 7.4 / 7.5, 8192^2 11.6 / 12.4, 22528 x
